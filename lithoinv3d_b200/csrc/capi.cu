@@ -158,12 +158,12 @@ struct lf_ctx {
     int dropCollapsed = 0;  // lf_set_collapsed_facets
     int xyMode = 0;
     double xyStep = 0.5;
-    DevBuf<double> d_fcfd;  // [7][NFC][nGradFacets] moved-facet constants
+    DevBuf<double> d_fcfd;  // [nGradFacets][7][NFC] moved-facet records
 
     // forward chunking (plan cached per station count and group filter;
     // uploaded only when it changes)
     std::vector<int32_t> chunkBegin, chunkEnd, chunkGroup;
-    int chunkCapacityS = 0, chunkFilter = -1, groupFilter = -1;
+    int chunkCapacityS = 0, chunkFilter = -1, groupFilter = -1, chunkLeast = 0;
     int64_t chunkFacets = 0;
     bool chunksDirty = true;
 
@@ -1052,6 +1052,8 @@ static constexpr int kFacetStage = 32;  // facet records per shared-memory stage
 static constexpr int kGradThreads = 32;             // Jacobian rows: one warp of facets per CTA
 static constexpr int kGradWarpsPerBlock = 4;        // objective gradient: one warp per facet
 
+constexpr int kFwdResident = 148 * 5;  // CTAs of k_forward_fp64 the GPU holds at once
+
 // Forward CTAs per launch of the chunked and item schedules; 0 (the mixed
 // path's persistent schedule) counts as 148 x 8 there.
 static int fwd_blocks(const lf_ctx* c) { return c->tune.fwd_target_blocks > 0 ? c->tune.fwd_target_blocks : 148 * 8; }
@@ -1059,15 +1061,21 @@ static int fwd_blocks(const lf_ctx* c) { return c->tune.fwd_target_blocks > 0 ? 
 // Facet chunks for the forward: contiguous ranges inside one group, sized so
 // that station tiles x chunks fill the GPU.
 // With c->groupFilter >= 0 only that group's facets are planned (unit
-// responses).
-static void plan_chunks(lf_ctx* c, int S) {
-    if (c->chunkCapacityS == S && c->chunkFilter == c->groupFilter && !c->chunksDirty && !c->chunkBegin.empty())
-        return;
+// responses).  Least facets per chunk: FP64, as many as one resident CTA of
+// k_forward_fp64 gets when the whole launch is resident at once, between 4
+// and 32 (a 320-facet body under 529 stations: 30 us at 64 facets, 10 us at 4;
+// 9,900 facets under 2,964 stations: 330, 316, 308 us at 128, 64, 32); mixed,
+// 64 (two full shared-memory stages).
+static void plan_chunks(lf_ctx* c, int S, bool fp64) {
     const int g0 = c->groupFilter >= 0 ? c->groupFilter : 0, g1 = c->groupFilter >= 0 ? c->groupFilter + 1 : c->G;
     const int nf = c->grpTriOff[g1] - c->grpTriOff[g0];
     int sBlocks = std::max(1, cdiv(S, kFwdThreads));
     int want = std::max(1, cdiv(fwd_blocks(c), sBlocks));
-    int chunkSize = std::max(64, cdiv(std::max(nf, 1), want));
+    const int least = fp64 ? std::min(32, std::max(4, cdiv((long long)nf * sBlocks, kFwdResident))) : 64;
+    if (c->chunkCapacityS == S && c->chunkFilter == c->groupFilter && c->chunkLeast == least && !c->chunksDirty &&
+        !c->chunkBegin.empty())
+        return;
+    int chunkSize = std::max(least, cdiv(std::max(nf, 1), want));
     c->chunkBegin.clear(); c->chunkEnd.clear(); c->chunkGroup.clear();
     for (int g = g0; g < g1; ++g)
         for (int f = c->grpTriOff[g]; f < c->grpTriOff[g + 1]; f += chunkSize) {
@@ -1077,6 +1085,7 @@ static void plan_chunks(lf_ctx* c, int S) {
         }
     c->chunkCapacityS = S;
     c->chunkFilter = c->groupFilter;
+    c->chunkLeast = least;
     c->chunkFacets = nf;
     c->chunksDirty = true;
     c->epoch++;
@@ -1221,7 +1230,7 @@ static lf_status forward_set_items(lf_ctx* c, const StationSet& s, double* d_gz,
                 TMI ? c->d_partM.p : nullptr, c->d_nearPairs.p);
         else
             k_forward_fp64_items<GZ, TMI, kFwdFacetTile><<<grid, kFwdThreads, 0, c->stream>>>(
-                c->d_items.p, c->nItems, s.d_xyz.p, c->T, c->d_fc.p, GZ ? c->d_partG.p : nullptr,
+                c->d_items.p, c->nItems, s.d_xyz.p, c->d_fc.p, GZ ? c->d_partG.p : nullptr,
                 TMI ? c->d_partM.p : nullptr);
         prof_end(c, c->evFwd, slot);
     }
@@ -1239,7 +1248,7 @@ static lf_status forward_set(lf_ctx* c, const StationSet& s, double* d_gz, doubl
     if (c->partitioned) return forward_set_items<GZ, TMI, false>(c, s, d_gz, d_tmi);
     int S = s.n;
     if (S == 0) return LF_OK;
-    plan_chunks(c, S);
+    plan_chunks(c, S, true);
     lf_status st = upload_chunks(c);
     if (st != LF_OK) return st;
     int nch = static_cast<int>(c->chunkBegin.size());
@@ -1249,7 +1258,7 @@ static lf_status forward_set(lf_ctx* c, const StationSet& s, double* d_gz, doubl
         dim3 grid(cdiv(S, kFwdThreads), nch);
         int slot = prof_begin(c, c->evFwd, c->nFwd);
         k_forward_fp64<GZ, TMI, kFwdFacetTile><<<grid, kFwdThreads, 0, c->stream>>>(
-            S, s.d_xyz.p, c->T, c->d_fc.p, c->d_chunkBegin.p, c->d_chunkEnd.p, GZ ? c->d_partG.p : nullptr,
+            S, s.d_xyz.p, c->d_fc.p, c->d_chunkBegin.p, c->d_chunkEnd.p, GZ ? c->d_partG.p : nullptr,
             TMI ? c->d_partM.p : nullptr);
         prof_end(c, c->evFwd, slot);
     }
@@ -1481,7 +1490,7 @@ static lf_status forward_set_facet(lf_ctx* c, const StationSet& s, double* d_gz,
     if (c->partitioned) return forward_set_items<GZ, TMI, true>(c, s, d_gz, d_tmi);
     int S = s.n;
     if (S == 0) return LF_OK;
-    plan_chunks(c, S);
+    plan_chunks(c, S, false);
     LF_RET_IF(upload_chunks(c));
     int nch = static_cast<int>(c->chunkBegin.size());
     if (GZ) LF_TRY_CUDA(c, c->d_partG.reserve((size_t)nch * S));

@@ -80,34 +80,17 @@ __global__ void k_na_prep(int nv, const double* __restrict__ xyz, int nt, const 
     if (f >= nt) return;
     int ia = tri[3 * f], ib = tri[3 * f + 1], ic = tri[3 * f + 2];
     double out[NFC];
-    for (int k = 0; k < NFC; ++k) out[k] = 0.0;
     if (ia < 0 || ia >= nv || ib < 0 || ib >= nv || ic < 0 || ic >= nv) {
         atomicExch(err, 1);
+        for (int k = 0; k < NFC; ++k) out[k] = 0.0;
+        out[FC_AREA2] = -1.0;
     } else {
-        d3 v[3] = {mk3(xyz[3 * ia], xyz[3 * ia + 1], xyz[3 * ia + 2]), mk3(xyz[3 * ib], xyz[3 * ib + 1], xyz[3 * ib + 2]),
-                   mk3(xyz[3 * ic], xyz[3 * ic + 1], xyz[3 * ic + 2])};
-        d3 n = cross_rn(sub_rn(v[1], v[0]), sub_rn(v[2], v[0]));
-        double area2 = norm_rn(n);
-        bool valid = !(area2 < kEps);
-        d3 un = valid ? div_rn(n, area2) : mk3(0, 0, 0);
-        out[FC_AX] = v[0].x; out[FC_AY] = v[0].y; out[FC_AZ] = v[0].z;
-        out[FC_BX] = v[1].x; out[FC_BY] = v[1].y; out[FC_BZ] = v[1].z;
-        out[FC_CX] = v[2].x; out[FC_CY] = v[2].y; out[FC_CZ] = v[2].z;
-        out[FC_NX] = un.x; out[FC_NY] = un.y; out[FC_NZ] = un.z;
-        out[FC_MF] = __dmul_rn(dot_rn(g.mdir, un), dot_rn(g.fdir, un));
-        for (int i = 0; i < 3; ++i) {
-            d3 e = sub_rn(v[(i + 1) % 3], v[i]);
-            double L = norm_rn(e);
-            d3 eh = (L < kEps) ? mk3(0, 0, 0) : div_rn(e, L);
-            d3 perp = cross_rn(un, eh);
-            out[FC_E0X + 3 * i] = e.x; out[FC_E0Y + 3 * i] = e.y; out[FC_E0Z + 3 * i] = e.z;
-            out[FC_L0 + i] = L;
-            out[FC_P0X + 3 * i] = perp.x; out[FC_P0Y + 3 * i] = perp.y; out[FC_P0Z + 3 * i] = perp.z;
-            out[FC_MT0 + i] = __dmul_rn(dot_rn(g.mdir, perp), dot_rn(g.fdir, perp));
-        }
-        out[FC_VALID] = valid ? 1.0 : 0.0;
+        const d3 v[3] = {mk3(xyz[3 * ia], xyz[3 * ia + 1], xyz[3 * ia + 2]),
+                         mk3(xyz[3 * ib], xyz[3 * ib + 1], xyz[3 * ib + 2]),
+                         mk3(xyz[3 * ic], xyz[3 * ic + 1], xyz[3 * ic + 2])};
+        face_consts_fwd(v, g.mdir, g.fdir, out);
     }
-    for (int k = 0; k < NFC; ++k) fc[(size_t)k * nt + f] = out[k];
+    store_face_fwd(out, fc + (size_t)f * NFC);
 }
 
 // Station-tiled pair kernel over uniform facet chunks of `cs` facets.
@@ -116,28 +99,12 @@ __global__ void __launch_bounds__(128) k_na_forward(int ns, const double* __rest
                                                     const double* __restrict__ fc, double* __restrict__ part_gz,
                                                     double* __restrict__ part_tmi) {
     using namespace litho_b200;
-    __shared__ double sm[NFC * FT];
+    __shared__ __align__(16) double sm[NFC * FT];
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     int chunk = blockIdx.y;
     int fb = chunk * cs, fe = min(nt, fb + cs);
-    d3 o = mk3(0, 0, 0);
-    if (s < ns) o = mk3(sta[3 * s], sta[3 * s + 1], sta[3 * s + 2]);
-    double gz = 0.0, tmi = 0.0;
-    for (int f0 = fb; f0 < fe; f0 += FT) {
-        int nf = min(FT, fe - f0);
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < NFC * FT; idx += blockDim.x) {
-            int k = idx / FT, j = idx % FT;
-            sm[idx] = (j < nf) ? fc[(size_t)k * nt + f0 + j] : 0.0;
-        }
-        __syncthreads();
-        if (s < ns)
-            for (int j = 0; j < nf; ++j) pair_forward_fp64<true, true>(sm, j, FT, o, &gz, &tmi);
-    }
-    if (s < ns) {
-        part_gz[(size_t)chunk * ns + s] = gz;
-        part_tmi[(size_t)chunk * ns + s] = tmi;
-    }
+    forward_fp64_block<true, true, FT>(sm, s, s < ns, sta, fc, fb, fe, part_gz + (size_t)chunk * ns,
+                                       part_tmi + (size_t)chunk * ns);
 }
 
 __global__ void k_na_reduce(int ns, int nch, const double* __restrict__ part_gz, const double* __restrict__ part_tmi,
@@ -163,10 +130,12 @@ extern "C" lf_status lf_forward_noalloc(int nv, const double* d_xyz, int nt, con
     if (!std::isfinite(density_gcc) || !std::isfinite(susceptibility_si) || !std::isfinite(inc_deg) ||
         !std::isfinite(dec_deg) || !std::isfinite(field_nt))
         return LF_EINVAL;
-    // Scratch layout (doubles): [0, 32) error flag and padding, facet constants
-    // NFC * nt, then gz and TMI chunk partials 2 * nch * ns.
+    // Scratch layout (doubles): [0, 32) error flag and padding, 38 per facet
+    // (the documented limit; its record takes the first NFC * nt of them),
+    // then gz and TMI chunk partials 2 * nch * ns.
     const size_t head = 32;
-    const size_t fcSize = (size_t)litho_b200::NFC * nt;
+    static_assert(litho_b200::NFC <= 38, "the documented size limit counts 38 doubles per facet");
+    const size_t fcSize = (size_t)38 * nt;
     if (head + fcSize + 2 * (size_t)ns > kNoallocScratchDoubles) return LF_EINVAL;
     const size_t room = (kNoallocScratchDoubles - head - fcSize) / (2 * (size_t)ns);
     int sBlocks = (ns + 127) / 128;
