@@ -355,6 +355,15 @@ __device__ __forceinline__ double rcp_pos64(double x) {
     return fma(y, fma(e, e, e), y);
 }
 
+// Square root of x > 0 and its reciprocal from one approximation.
+__device__ __forceinline__ double sqrt_inv64(double x, double* inv) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double t = x * y, e = fma(-t, y, 1.0), ep = e * fma(0.375, e, 0.5);
+    *inv = fma(y, ep, y);
+    return fma(t, ep, t);
+}
+
 // atanh(v) for 0 <= v <= 1/2 (atanh_poly64), for v <= 1/4 (atanh_short64), and
 // atan(t) for t^2 <= 0.1: polynomials in the square, Chebyshev interpolants of
 // atanh(sqrt w) / sqrt w on [0, 1/4] and [0, 1/16] and of atan(sqrt w) /
@@ -735,26 +744,11 @@ struct GradAcc {
     double alam[3];     // sum Gs * Lambda_i       (d_perp direct on p1)
     double aom;         // sum Gs * Omega          (h direct on a)
     double ai;          // sum G0 * I              (n_z factor)
-    d3 bh;              // sum Gs * Omega * r_a    (h through n_hat)
-    d3 bl[3];           // sum Gs * Lambda_i * r1  (d_perp through perp_i)
+    d3 bh;              // sum Gs * Omega * r_a    (h through n_hat; z is not needed)
+    d3 bl[3];           // sum Gs * Lambda_i * r1  (d_perp through perp_i; bl[0].y is not needed)
     double amf;         // sum Ts * Omega          (MF)
     double amt[3];      // sum Ts * Lambda_i       (MT_i)
 };
-
-__device__ __forceinline__ void edge_terms(d3 r1, d3 r2, double d1, double d2, double ex, double ey, double L,
-                                           double inv1, double inv2, double kom, double Gs, double Ts, double mt,
-                                           double dperp, double lam, bool live, d3* g1, d3* g2) {
-    // kappa_i = Gs * d_perp + Ts * MT_i
-    double kl = live ? (Gs * dperp + Ts * mt) : 0.0;
-    double dw = d1 * d2 + dot3(r1, r2);
-    double W = dw > 1e-300 ? L / dw : 0.0;
-    double s1 = r1.x * ex + r1.y * ey;
-    d3 q = mk3(r1.x - s1 * ex, r1.y - s1 * ey, r1.z);
-    d3 Z = mk3(ey * r1.z, -ex * r1.z, ex * r1.y - ey * r1.x);  // e_hat x r1, e_hat = (ex, ey, 0)
-    d3 P = mk3(W * (kom * Z.x - kl * q.x), W * (kom * Z.y - kl * q.y), W * (kom * Z.z - kl * q.z));
-    *g1 = *g1 + mk3((P.x - kl * ex) * inv1, (P.y - kl * ey) * inv1, P.z * inv1);
-    *g2 = *g2 + mk3((P.x + kl * ex) * inv2, (P.y + kl * ey) * inv2, P.z * inv2);
-}
 
 // Per-facet finalisation in the local frame: differentiates the facet
 // constants (n_z, the unit normal, the in-plane edge normals, the magnetic
@@ -853,56 +847,154 @@ __device__ __forceinline__ bool tile_far(const FarKey& k, const double* __restri
     return dd >= k.th2;
 }
 
+// Omega, the edge integrals, W_i = L_i / (d1 d2 + r1.r2) and which edges are
+// live (bit i) for a pair close to its facet, by the library functions; dead:
+// the station lies on a vertex, where nothing is differentiable.
+struct NearTerms {
+    double om, lam[3], W[3];
+    int live;
+    bool dead;
+};
+__device__ __forceinline__ NearTerms gradient_near_terms(double x, double y, double z, double L0, double cx, double cy,
+                                                      double L1, double L2) {
+    NearTerms N;
+    const d3 r[3] = {mk3(-x, -y, -z), mk3(L0 - x, -y, -z), mk3(cx - x, cy - y, -z)};
+    double l[3];
+    N.dead = false;
+    N.live = 0;
+    for (int i = 0; i < 3; ++i) {
+        l[i] = sqrt(dot3(r[i], r[i]));
+        N.dead |= l[i] < kEps;
+    }
+    const double L[3] = {L0, L1, L2};
+    double den = l[0] * l[1] * l[2];
+    for (int i = 0; i < 3; ++i) {
+        const int j = (i + 1) % 3;
+        const double dot = dot3(r[i], r[j]), dw = l[i] * l[j] + dot;
+        bool lv;
+        N.lam[i] = lambda_sym(l[i], l[j], L[i], &lv);
+        N.live |= lv ? 1 << i : 0;
+        N.W[i] = dw > 1e-300 ? L[i] / dw : 0.0;
+        den += dot * l[(i + 2) % 3];
+    }
+    N.om = 2.0 * atan2(-z * (L0 * cy), den);
+    return N;
+}
+
 // One (facet, station) pair of the FP64 gradient: adds the station's terms,
 // weighted by its adjoints (gco gravity, mco magnetic), to the facet's
 // local-frame accumulators.  gsn / ms: the facet group's gz / TMI scales.
+// GZ / TMI: which adjoints can be non-zero.
+//
+// Per edge with direction e, in-plane normal n = (-ey, ex), kl = Gs d_perp +
+// Ts MT and kom = -Gs h + Ts MF, the vertex terms are
+//   p1 += (-kl e + alpha n + beta z) / d1,  p2 += (kl e + alpha n + beta z) / d2,
+//   alpha = W (kom z + kl d_perp),  beta = W (kl z - kom d_perp),
+// (q = r1 - (r1.e) e = -d_perp n - z zhat and e x r1 = z n - d_perp zhat in
+// the facet's frame), so the terms of a vertex's two edges are added before
+// the division by its distance.  Away from the facet (every v = L / (d1 + d2)
+// below 1/2, see pair_forward_fp64) 1 / (d1 + d2) and W = 2 L / ((d1 + d2)^2 -
+// L^2) share one reciprocal and the polynomials replace the library's log1p
+// and atan2; other pairs take gradient_near_terms.  233 FP64 instructions per
+// pair (ncu) against more than 700 through the library functions.
+template <bool GZ, bool TMI>
 __device__ __forceinline__ void pair_gradient_fp64(const double* C, double gsn, double ms, double ox, double oy,
                                                    double oz, double gco, double mco, GradAcc& A) {
-    const double nz = C[GC_ZZ];
-    const double L0 = C[GC_L0], cx = C[GC_CX], cy = C[GC_CY];
-    const double area2 = L0 * cy;
-    double G0 = gco * gsn;  // gravity adjoint x group scale
-    double Gs = G0 * nz;    // ... x n_z
-    double Ts = mco * ms;   // magnetic adjoint x group TMI scale
-    if (Gs == 0.0 && Ts == 0.0 && G0 == 0.0) return;
-    d3 dd = mk3(ox - C[GC_AX], oy - C[GC_AY], oz - C[GC_AZ]);
-    double x = dd.x * C[GC_XX] + dd.y * C[GC_XY] + dd.z * C[GC_XZ];
-    double y = dd.x * C[GC_YX] + dd.y * C[GC_YY] + dd.z * C[GC_YZ];
-    double z = dd.x * C[GC_ZX] + dd.y * C[GC_ZY] + dd.z * C[GC_ZZ];
-    d3 ra = mk3(-x, -y, -z), rb = mk3(L0 - x, -y, -z), rc = mk3(cx - x, cy - y, -z);
-    double z2 = z * z;
-    double la = sqrt(x * x + y * y + z2), lb = sqrt(rb.x * rb.x + y * y + z2),
-           lc = sqrt(rc.x * rc.x + rc.y * rc.y + z2);
-    if (la < kEps || lb < kEps || lc < kEps) return;  // station on a vertex: not differentiable
-    double h = -z;
-    double Nn = h * area2;
-    double Dd = la * lb * lc + dot3(ra, rb) * lc + dot3(ra, rc) * lb + dot3(rb, rc) * la;
-    double om = 2.0 * atan2(Nn, Dd);
-    double ia = 1.0 / la, ib = 1.0 / lb, ic = 1.0 / lc;
-    // edges: 0 a->b (e=(1,0)), 1 b->c, 2 c->a
-    double e1x = C[GC_E1X], e1y = C[GC_E1Y], e2x = C[GC_E2X], e2y = C[GC_E2Y];
-    bool lv0, lv1, lv2;
-    double lam0 = lambda_sym(la, lb, L0, &lv0);
-    double lam1 = lambda_sym(lb, lc, C[GC_L1], &lv1);
-    double lam2 = lambda_sym(lc, la, C[GC_L2], &lv2);
-    // d_perp_i = -r1 . perp_i, perp_i = (-ey, ex, 0)
-    double dp0 = y;  // -(r_a.y * 1)
-    double dp1 = rb.x * e1y - rb.y * e1x;
-    double dp2 = rc.x * e2y - rc.y * e2x;
-    double I = dp0 * lam0 + dp1 * lam1 + dp2 * lam2 - h * om;
-    double kom = -Gs * h + Ts * C[GC_MF];
-    edge_terms(ra, rb, la, lb, 1.0, 0.0, L0, ia, ib, kom, Gs, Ts, C[GC_MT0], dp0, lam0, lv0, &A.va, &A.vb);
-    edge_terms(rb, rc, lb, lc, e1x, e1y, C[GC_L1], ib, ic, kom, Gs, Ts, C[GC_MT1], dp1, lam1, lv1, &A.vb, &A.vc);
-    edge_terms(rc, ra, lc, la, e2x, e2y, C[GC_L2], ic, ia, kom, Gs, Ts, C[GC_MT2], dp2, lam2, lv2, &A.vc, &A.va);
-    A.alam[0] += Gs * lam0; A.alam[1] += Gs * lam1; A.alam[2] += Gs * lam2;
-    A.aom += Gs * om;
-    A.ai += G0 * I;
-    A.bh = A.bh + ra * (Gs * om);
-    A.bl[0] = A.bl[0] + ra * (Gs * lam0);
-    A.bl[1] = A.bl[1] + rb * (Gs * lam1);
-    A.bl[2] = A.bl[2] + rc * (Gs * lam2);
-    A.amf += Ts * om;
-    A.amt[0] += Ts * lam0; A.amt[1] += Ts * lam1; A.amt[2] += Ts * lam2;
+    const double L0 = C[GC_L0], cx = C[GC_CX], cy = C[GC_CY], L1 = C[GC_L1], L2 = C[GC_L2];
+    const double G0 = GZ ? gco * gsn : 0.0;      // gravity adjoint x group scale
+    const double Gs = GZ ? G0 * C[GC_ZZ] : 0.0;  // ... x n_z
+    const double Ts = TMI ? mco * ms : 0.0;      // magnetic adjoint x group TMI scale
+    if (G0 == 0.0 && Ts == 0.0) return;
+    const d3 dd = mk3(ox - C[GC_AX], oy - C[GC_AY], oz - C[GC_AZ]);
+    const double x = dd.x * C[GC_XX] + dd.y * C[GC_XY] + dd.z * C[GC_XZ];
+    const double y = dd.x * C[GC_YX] + dd.y * C[GC_YY] + dd.z * C[GC_YZ];
+    const double z = dd.x * C[GC_ZX] + dd.y * C[GC_ZY] + dd.z * C[GC_ZZ];
+    const double rbx = L0 - x, rcx = cx - x, rcy = cy - y;
+    const double z2 = z * z, yz2 = fma(y, y, z2);
+    const double a2 = fma(x, x, yz2), b2 = fma(rbx, rbx, yz2), c2 = fma(rcx, rcx, fma(rcy, rcy, z2));
+    double ia, ib, ic;
+    const double la = sqrt_inv64(a2, &ia), lb = sqrt_inv64(b2, &ib), lc = sqrt_inv64(c2, &ic);
+    const double D0 = la + lb, D1 = lb + lc, D2 = lc + la;
+    const double m0 = fma(D0, D0, -L0 * L0), m1 = fma(D1, D1, -L1 * L1), m2 = fma(D2, D2, -L2 * L2);
+    const double g0 = rcp_pos64(D0 * m0), g1 = rcp_pos64(D1 * m1), g2 = rcp_pos64(D2 * m2);
+    const double v0 = L0 * (g0 * m0), v1 = L1 * (g1 * m1), v2 = L2 * (g2 * m2);
+    const int vmax = max(__double2hiint(v0), max(__double2hiint(v1), __double2hiint(v2)));
+    double om, l0, l1, l2, W0, W1, W2;
+    bool lv0 = true, lv1 = true, lv2 = true;
+    if (vmax < 0x3fe00000) {  // every v < 1/2
+        W0 = (L0 + L0) * (g0 * D0);
+        W1 = (L1 + L1) * (g1 * D1);
+        W2 = (L2 + L2) * (g2 * D2);
+        // ra . rb = (a2 + b2 - L^2) / 2
+        const double dab = 0.5 * fma(-L0, L0, a2 + b2), dbc = 0.5 * fma(-L1, L1, b2 + c2),
+                     dac = 0.5 * fma(-L2, L2, c2 + a2);
+        const double den = fma(la * lb, lc, fma(dab, lc, fma(dac, lb, dbc * la)));
+        om = 2.0 * atan_poly64(-z * (L0 * cy) * rcp_pos64(den));
+        if (vmax < 0x3fd00000) {  // every v < 1/4
+            l0 = 2.0 * atanh_short64(v0);
+            l1 = 2.0 * atanh_short64(v1);
+            l2 = 2.0 * atanh_short64(v2);
+        } else {
+            l0 = 2.0 * atanh_poly64(v0);
+            l1 = 2.0 * atanh_poly64(v1);
+            l2 = 2.0 * atanh_poly64(v2);
+        }
+    } else {
+        const NearTerms N = gradient_near_terms(x, y, z, L0, cx, cy, L1, L2);
+        if (N.dead) return;
+        om = N.om;
+        l0 = N.lam[0]; l1 = N.lam[1]; l2 = N.lam[2];
+        W0 = N.W[0]; W1 = N.W[1]; W2 = N.W[2];
+        lv0 = N.live & 1; lv1 = N.live & 2; lv2 = N.live & 4;
+    }
+    // edges: 0 a->b (e = (1, 0)), 1 b->c, 2 c->a
+    const double e1x = C[GC_E1X], e1y = C[GC_E1Y], e2x = C[GC_E2X], e2y = C[GC_E2Y];
+    const double dp0 = y, dp1 = fma(rbx, e1y, y * e1x), dp2 = fma(rcx, e2y, -rcy * e2x);  // -r1 . n_i
+    double kom, k0, k1, k2;
+    if (TMI) {
+        kom = Ts * C[GC_MF];
+        k0 = Ts * C[GC_MT0];
+        k1 = Ts * C[GC_MT1];
+        k2 = Ts * C[GC_MT2];
+    }
+    if (GZ) {
+        kom = TMI ? fma(Gs, z, kom) : Gs * z;
+        k0 = TMI ? fma(Gs, dp0, k0) : Gs * dp0;
+        k1 = TMI ? fma(Gs, dp1, k1) : Gs * dp1;
+        k2 = TMI ? fma(Gs, dp2, k2) : Gs * dp2;
+    }
+    if (!lv0) k0 = 0.0;
+    if (!lv1) k1 = 0.0;
+    if (!lv2) k2 = 0.0;
+    const double kz = kom * z;
+    const double al0 = W0 * fma(k0, dp0, kz), be0 = W0 * fma(k0, z, -kom * dp0);
+    const double al1 = W1 * fma(k1, dp1, kz), be1 = W1 * fma(k1, z, -kom * dp1);
+    const double al2 = W2 * fma(k2, dp2, kz), be2 = W2 * fma(k2, z, -kom * dp2);
+    A.va.x = fma(ia, fma(-al2, e2y, fma(k2, e2x, -k0)), A.va.x);
+    A.va.y = fma(ia, fma(al2, e2x, fma(k2, e2y, al0)), A.va.y);
+    A.va.z = fma(ia, be0 + be2, A.va.z);
+    A.vb.x = fma(ib, fma(-al1, e1y, fma(-k1, e1x, k0)), A.vb.x);
+    A.vb.y = fma(ib, fma(al1, e1x, fma(-k1, e1y, al0)), A.vb.y);
+    A.vb.z = fma(ib, be0 + be1, A.vb.z);
+    A.vc.x = fma(ic, fma(-al2, e2y, fma(-k2, e2x, fma(-al1, e1y, k1 * e1x))), A.vc.x);
+    A.vc.y = fma(ic, fma(al2, e2x, fma(-k2, e2y, fma(al1, e1x, k1 * e1y))), A.vc.y);
+    A.vc.z = fma(ic, be1 + be2, A.vc.z);
+    if (GZ) {
+        const double w0 = Gs * l0, w1 = Gs * l1, w2 = Gs * l2, wo = Gs * om;
+        A.ai = fma(G0, fma(dp0, l0, fma(dp1, l1, fma(dp2, l2, z * om))), A.ai);
+        A.alam[0] += w0; A.alam[1] += w1; A.alam[2] += w2;
+        A.aom += wo;
+        A.bh.x = fma(-x, wo, A.bh.x); A.bh.y = fma(-y, wo, A.bh.y);
+        A.bl[0].x = fma(-x, w0, A.bl[0].x); A.bl[0].z = fma(-z, w0, A.bl[0].z);
+        A.bl[1].x = fma(rbx, w1, A.bl[1].x); A.bl[1].y = fma(-y, w1, A.bl[1].y); A.bl[1].z = fma(-z, w1, A.bl[1].z);
+        A.bl[2].x = fma(rcx, w2, A.bl[2].x); A.bl[2].y = fma(rcy, w2, A.bl[2].y); A.bl[2].z = fma(-z, w2, A.bl[2].z);
+    }
+    if (TMI) {
+        A.amf = fma(Ts, om, A.amf);
+        A.amt[0] = fma(Ts, l0, A.amt[0]);
+        A.amt[1] = fma(Ts, l1, A.amt[1]);
+        A.amt[2] = fma(Ts, l2, A.amt[2]);
+    }
 }
 
 __device__ __forceinline__ bool facet_grad_active(const double* C) {
@@ -934,7 +1026,7 @@ __global__ void __launch_bounds__(32) k_gradient_fp64(int T, const double* __res
         grad_acc_zero(A);
         const double gsn = C[GC_GS], ms = C[GC_MS];
         for (int j = sb; j < se; ++j)
-            pair_gradient_fp64(C, gsn, ms, sta[3 * j], sta[3 * j + 1], sta[3 * j + 2], gcoef ? gcoef[j] : 0.0,
+            pair_gradient_fp64<true, true>(C, gsn, ms, sta[3 * j], sta[3 * j + 1], sta[3 * j + 2], gcoef ? gcoef[j] : 0.0,
                                mcoef ? mcoef[j] : 0.0, A);
         grad_finalize(C, A, groups[face_group[f]], fdir, outv);
     }
@@ -947,20 +1039,42 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-__device__ __forceinline__ void grad_acc_warp_sum(GradAcc& A) {
-    A.va = mk3(warp_sum(A.va.x), warp_sum(A.va.y), warp_sum(A.va.z));
-    A.vb = mk3(warp_sum(A.vb.x), warp_sum(A.vb.y), warp_sum(A.vb.z));
-    A.vc = mk3(warp_sum(A.vc.x), warp_sum(A.vc.y), warp_sum(A.vc.z));
-    A.bh = mk3(warp_sum(A.bh.x), warp_sum(A.bh.y), warp_sum(A.bh.z));
+// Warp totals of the accumulators, transposed: 28 sums padded to 32 are folded
+// in five halving steps (31 exchanges instead of 28 x 5), lane k writes total
+// k to row[k] (shared memory, 32 doubles), and every lane reads them back.
+__device__ __forceinline__ void grad_acc_warp_sum(GradAcc& A, double* row) {
+    const int lane = threadIdx.x & 31;
+    double v[32] = {A.va.x, A.va.y, A.va.z, A.vb.x, A.vb.y, A.vb.z, A.vc.x, A.vc.y, A.vc.z,
+                    A.bh.x, A.bh.y, A.bl[0].x, A.bl[0].z, A.bl[1].x, A.bl[1].y, A.bl[1].z,
+                    A.bl[2].x, A.bl[2].y, A.bl[2].z, A.alam[0], A.alam[1], A.alam[2], A.aom, A.ai,
+                    A.amf, A.amt[0], A.amt[1], A.amt[2], 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1) {
+        const bool upper = (lane & step) != 0;
+#pragma unroll
+        for (int i = 0; i < step; ++i) {
+            const double send = upper ? v[i] : v[i + step];
+            const double keep = upper ? v[i + step] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, step);
+        }
+    }
+    row[lane] = v[0];
+    __syncwarp();
+    A.va = mk3(row[0], row[1], row[2]);
+    A.vb = mk3(row[3], row[4], row[5]);
+    A.vc = mk3(row[6], row[7], row[8]);
+    A.bh = mk3(row[9], row[10], 0.0);
+    A.bl[0] = mk3(row[11], 0.0, row[12]);
+    A.bl[1] = mk3(row[13], row[14], row[15]);
+    A.bl[2] = mk3(row[16], row[17], row[18]);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        A.alam[i] = warp_sum(A.alam[i]);
-        A.amt[i] = warp_sum(A.amt[i]);
-        A.bl[i] = mk3(warp_sum(A.bl[i].x), warp_sum(A.bl[i].y), warp_sum(A.bl[i].z));
+        A.alam[i] = row[19 + i];
+        A.amt[i] = row[25 + i];
     }
-    A.aom = warp_sum(A.aom);
-    A.ai = warp_sum(A.ai);
-    A.amf = warp_sum(A.amf);
+    A.aom = row[22];
+    A.ai = row[23];
+    A.amf = row[24];
 }
 
 // Objective gradient, FP64: one warp per facet.  The warp visits the
@@ -971,6 +1085,11 @@ __device__ __forceinline__ void grad_acc_warp_sum(GradAcc& A) {
 // Warps run over `facets` (those with a DOF vertex); grid.y splits the
 // station tiles into chunks of tiles_per_chunk so that a model with few such
 // facets still fills the GPU.  part layout [chunk][9][T].
+// FP64 pipe 65 % busy at 12 warps per SM (168 registers, of which 56 hold the
+// sums): 24.6 M pairs (8,308 facets, 2,964 stations) took 1,131 us with the
+// library functions, 489 us now; a 1,280-facet body under 1,600 stations 115
+// and 57 us.  Two CTAs per SM (no spill) 523 us, four (128 registers) 539;
+// CTAs of one or two warps no different.
 __global__ void __launch_bounds__(128, 3) k_gradient_warp_fp64(int T, const double* __restrict__ gc, int S,
                                                             const double* __restrict__ sta,
                                                             const double* __restrict__ gcoef,
@@ -999,7 +1118,7 @@ __global__ void __launch_bounds__(128, 3) k_gradient_warp_fp64(int T, const doub
     part += (size_t)blockIdx.y * 9 * T;
     // the facet's constants live in shared memory (one row per warp): the
     // per-lane FP64 sums and pair temporaries need the registers
-    __shared__ double Csh[4][NGC];
+    __shared__ double Csh[4][NGC], sums[4][32];
     double* C = Csh[threadIdx.x >> 5];
     if (lane < NGC) C[lane] = gc[(size_t)lane * T + f];
     __syncwarp();
@@ -1023,13 +1142,13 @@ __global__ void __launch_bounds__(128, 3) k_gradient_warp_fp64(int T, const doub
                 for (int k = 0; k < kStationTile; k += 32) {
                     const int j = s0 + k + lane;
                     if (j < S)
-                        pair_gradient_fp64(C, gsn, ms, sta[3 * j], sta[3 * j + 1], sta[3 * j + 2],
+                        pair_gradient_fp64<true, true>(C, gsn, ms, sta[3 * j], sta[3 * j + 1], sta[3 * j + 2],
                                            gcoef ? gcoef[j] : 0.0, mcoef ? mcoef[j] : 0.0, A);
                 }
             }
         }
         if (any) {
-            grad_acc_warp_sum(A);
+            grad_acc_warp_sum(A, sums[threadIdx.x >> 5]);
             if (lane == 0) grad_finalize(C, A, groups[face_group[f]], fdir, outv);
         }
     }

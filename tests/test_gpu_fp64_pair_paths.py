@@ -8,7 +8,7 @@ s1 + d1 (stations at least 20 degrees off an edge's direction)."""
 import numpy as np
 import pytest
 
-from lithoinv3d_b200 import synth
+from lithoinv3d_b200 import GRAVITY, MAGNETIC, synth
 from oracle_bindings import OracleModel
 
 pytestmark = pytest.mark.gpu
@@ -71,3 +71,21 @@ def test_forward_routes(name):
     tol = 256 * EPS * term_sums(sta, 0.3, 0.02, p.inducing)
     assert np.all(np.abs(gz - om.forward_gz(sta)) <= tol[:, 0])
     assert np.all(np.abs(tmi - om.forward_tmi(sta)) <= tol[:, 1])
+
+
+@pytest.mark.parametrize("which", [GRAVITY, MAGNETIC])
+@pytest.mark.parametrize("name", ["quarter", "half", "close"])
+def test_derivative_routes(name, which):
+    """Jacobian rows on both sides of the lines between the routes, against the
+    oracle's central-difference truth (1e-6 of the row's largest entry, the
+    tolerance of the other Jacobian tests)."""
+    sta = CASES[name]
+    p = synth.Problem("tetrahedron", [0.3], [0.02], [(V, F, synth.XYZ_FREE)], sta, sta)
+    model = p.build_model()
+    ctx = p.make_context(model)
+    x = model.assemble_parameters()
+    J = ctx.jacobian(x, which)
+    om = OracleModel(model.tables(), p.densities, p.susceptibilities, p.inducing)
+    om.scatter(x)
+    Jt = om.jacobian(sta, 2 + which)
+    assert np.all(np.abs(J - Jt).max(1) <= 1e-6 * np.abs(Jt).max(1))
