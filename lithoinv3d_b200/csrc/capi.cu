@@ -164,6 +164,7 @@ struct lf_ctx {
     // uploaded only when it changes)
     std::vector<int32_t> chunkBegin, chunkEnd, chunkGroup;
     int chunkCapacityS = 0, chunkFilter = -1, groupFilter = -1, chunkLeast = 0;
+    int fp64Slices = 1;  // facet slices per CTA of the planned FP64 forward
     int64_t chunkFacets = 0;
     bool chunksDirty = true;
 
@@ -1061,17 +1062,25 @@ static int fwd_blocks(const lf_ctx* c) { return c->tune.fwd_target_blocks > 0 ? 
 // Facet chunks for the forward: contiguous ranges inside one group, sized so
 // that station tiles x chunks fill the GPU.
 // With c->groupFilter >= 0 only that group's facets are planned (unit
-// responses).  Least facets per chunk: FP64, as many as one resident CTA of
-// k_forward_fp64 gets when the whole launch is resident at once, between 4
-// and 32 (a 320-facet body under 529 stations: 30 us at 64 facets, 10 us at 4;
-// 9,900 facets under 2,964 stations: 330, 316, 308 us at 128, 64, 32); mixed,
-// 64 (two full shared-memory stages).
+// responses).  fp64: the plan of k_forward_fp64.  Least facets per chunk: 32
+// there (9,900 facets under 2,964 stations: 330, 316, 308 us at 128, 64, 32),
+// 64 in mixed precision (two full shared-memory stages).  An FP64 launch that
+// would not fill the GPU twice over at 32 facets takes the sliced form with
+// 32 stations per CTA and 16 to 32 facets per chunk (a 320-facet body under
+// 529 stations: 30 us with 64-facet chunks and 128 stations, 11 us now; finer
+// chunks instead of slices are as fast, but their partials cost a new
+// context's first call another 0.3 ms of allocation).
 static void plan_chunks(lf_ctx* c, int S, bool fp64) {
     const int g0 = c->groupFilter >= 0 ? c->groupFilter : 0, g1 = c->groupFilter >= 0 ? c->groupFilter + 1 : c->G;
     const int nf = c->grpTriOff[g1] - c->grpTriOff[g0];
     int sBlocks = std::max(1, cdiv(S, kFwdThreads));
     int want = std::max(1, cdiv(fwd_blocks(c), sBlocks));
-    const int least = fp64 ? std::min(32, std::max(4, cdiv((long long)nf * sBlocks, kFwdResident))) : 64;
+    int least = fp64 ? 32 : 64;
+    c->fp64Slices = 1;
+    if (fp64 && (long long)sBlocks * cdiv(nf, 32) < 2 * kFwdResident) {
+        c->fp64Slices = 4;
+        least = std::min(32, std::max(16, cdiv((long long)nf * cdiv(S, 32), kFwdResident)));
+    }
     if (c->chunkCapacityS == S && c->chunkFilter == c->groupFilter && c->chunkLeast == least && !c->chunksDirty &&
         !c->chunkBegin.empty())
         return;
@@ -1255,9 +1264,10 @@ static lf_status forward_set(lf_ctx* c, const StationSet& s, double* d_gz, doubl
     if (GZ) LF_TRY_CUDA(c, c->d_partG.reserve((size_t)nch * S));
     if (TMI) LF_TRY_CUDA(c, c->d_partM.reserve((size_t)nch * S));
     if (nch > 0) {
-        dim3 grid(cdiv(S, kFwdThreads), nch);
+        const bool sliced = c->fp64Slices > 1;
+        const auto kernel = sliced ? k_forward_fp64<GZ, TMI, kFwdFacetTile, 4> : k_forward_fp64<GZ, TMI, kFwdFacetTile, 1>;
         int slot = prof_begin(c, c->evFwd, c->nFwd);
-        k_forward_fp64<GZ, TMI, kFwdFacetTile><<<grid, kFwdThreads, 0, c->stream>>>(
+        kernel<<<dim3(cdiv(S, sliced ? 32 : kFwdThreads), nch), kFwdThreads, 0, c->stream>>>(
             S, s.d_xyz.p, c->d_fc.p, c->d_chunkBegin.p, c->d_chunkEnd.p, GZ ? c->d_partG.p : nullptr,
             TMI ? c->d_partM.p : nullptr);
         prof_end(c, c->evFwd, slot);

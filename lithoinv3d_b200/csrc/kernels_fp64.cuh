@@ -510,11 +510,16 @@ __device__ __forceinline__ void pair_forward_fp64(const double* __restrict__ F, 
     }
 }
 
-// Grid: x = station tiles of blockDim.x, y = facet chunks (each inside one
-// group).  Writes the chunk's unscaled facet sums per station.
+// Grid: x = station blocks, y = facet chunks (each inside one group).  Writes
+// the chunk's unscaled facet sums per station.
 // One CTA's work: station s (act = s is a station of the block) against
 // facets [fb, fe); out_gz[s] / out_tmi[s] receive the unscaled sums.
-template <bool GZ, bool TMI, int FT>
+// SLICES = 1: one station per thread of the CTA, every thread against every
+// facet.  SLICES = 4: the CTA's four warps hold the same 32 stations and take
+// every fourth facet each; their sums are added in warp order through shared
+// memory.  The second form gives a small launch four times the CTAs for the
+// same number of chunk partials.
+template <bool GZ, bool TMI, int FT, int SLICES = 1>
 __device__ __forceinline__ void forward_fp64_block(double* __restrict__ sm, int s, bool act,
                                                    const double* __restrict__ sta, const double* __restrict__ fc,
                                                    int fb, int fe, double* __restrict__ out_gz,
@@ -530,7 +535,20 @@ __device__ __forceinline__ void forward_fp64_block(double* __restrict__ sm, int 
             reinterpret_cast<double2*>(sm)[idx] = __ldg(src + idx);
         __syncthreads();
         if (act)
-            for (int j = 0; j < nf; ++j) pair_forward_fp64<GZ, TMI>(sm + j * NFC, o, &gz, &tmi);
+            for (int j = SLICES == 1 ? 0 : (int)(threadIdx.x >> 5); j < nf; j += SLICES)
+                pair_forward_fp64<GZ, TMI>(sm + j * NFC, o, &gz, &tmi);
+    }
+    if (SLICES > 1) {
+        __syncthreads();  // the records are no longer read
+        sm[threadIdx.x] = gz;
+        sm[blockDim.x + threadIdx.x] = tmi;
+        __syncthreads();
+        if (threadIdx.x >= 32) return;
+#pragma unroll
+        for (int k = 1; k < SLICES; ++k) {
+            gz += sm[32 * k + threadIdx.x];
+            tmi += sm[blockDim.x + 32 * k + threadIdx.x];
+        }
     }
     if (act) {
         if (GZ) out_gz[s] = gz;
@@ -542,17 +560,20 @@ __device__ __forceinline__ void forward_fp64_block(double* __restrict__ sm, int 
 // library functions and SoA records in shared memory, 291 us now, 1.0e11
 // pairs/s.  Five CTAs per SM: six or seven (84, 72 registers) are 3 and 6 %
 // slower, the unbounded 96 registers 2 %.
-template <bool GZ, bool TMI, int FT>
+template <bool GZ, bool TMI, int FT, int SLICES>
 __global__ void __launch_bounds__(128, 5) k_forward_fp64(int S, const double* __restrict__ sta,
-                                                      const double* __restrict__ fc, const int32_t* __restrict__ chunk_begin,
-                                                      const int32_t* __restrict__ chunk_end, double* __restrict__ part_gz,
-                                                      double* __restrict__ part_tmi) {
+                                                         const double* __restrict__ fc,
+                                                         const int32_t* __restrict__ chunk_begin,
+                                                         const int32_t* __restrict__ chunk_end,
+                                                         double* __restrict__ part_gz, double* __restrict__ part_tmi) {
     __shared__ __align__(16) double sm[NFC * FT];
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    static_assert(NFC * FT >= 2 * 128, "the slices' sums fit where the records were");
+    const int s = SLICES == 1 ? (int)(blockIdx.x * blockDim.x + threadIdx.x)
+                              : (int)(blockIdx.x * 32 + (threadIdx.x & 31));
     const int chunk = blockIdx.y;
-    forward_fp64_block<GZ, TMI, FT>(sm, s, s < S, sta, fc, chunk_begin[chunk], chunk_end[chunk],
-                                    GZ ? part_gz + (size_t)chunk * S : nullptr,
-                                    TMI ? part_tmi + (size_t)chunk * S : nullptr);
+    forward_fp64_block<GZ, TMI, FT, SLICES>(sm, s, s < S, sta, fc, chunk_begin[chunk], chunk_end[chunk],
+                                            GZ ? part_gz + (size_t)chunk * S : nullptr,
+                                            TMI ? part_tmi + (size_t)chunk * S : nullptr);
 }
 
 // Batched bodies: a persistent grid walks a list of (station block, facet
