@@ -112,6 +112,7 @@ struct lf_ctx {
     PatchTopology ptopo;
     DevBuf<int32_t> d_pFacetOff, d_pFacets, d_pVertOff, d_pVerts, d_pEdgeOff, d_pBlobOff, d_pChunkBegin, d_pChunkEnd,
         d_pFacetPatch, d_pFacetSlot;
+    DevBuf<float> d_adj32;  // far-field gradient: FP32 adjoints x group scales
     DevBuf<float> d_mt2;  // doubled TMI edge coefficients of every facet [3][T]
     DevBuf<uint32_t> d_pCorners, d_pEdgeInfo;
     DevBuf<uint8_t> d_pEdgeSlot, d_blobs;
@@ -1656,7 +1657,15 @@ static int grad_slots(lf_ctx* c, int S) {
     return n1;
 }
 
-// Gradient kernels over one station set with the given adjoints; writes
+// The FP32 adjoints of gradient_set's far-field kernel over S stations.
+static lf_status far_workspace(lf_ctx* c, int S) {
+    if (c->precision == LF_PREC_MIXED)
+        LF_TRY_CUDA(c, c->d_adj32.reserve(2 * (size_t)(c->partitioned ? 1 : c->G) * S));
+    return LF_OK;
+}
+
+// Gradient kernels over one station set with the given adjoints (after
+// far_workspace); writes
 // facet partial slots [slot0, slot0 + returned count) of d_partGrad
 // ([slot][9][T], one slot per (kernel, station chunk)).
 static int gradient_set(lf_ctx* c, const StationSet& s, const double* gcoef, const double* mcoef, int slot0) {
@@ -1688,9 +1697,16 @@ static int gradient_set(lf_ctx* c, const StationSet& s, const double* gcoef, con
         int nch2 = 1, tpc2 = 1;
         grad_chunks(c, s.n, false, &nch2, &tpc2);
         int ev2 = prof_begin(c, c->evGrad, c->nGrad);
-        k_gradient_warp_far32<<<dim3(fblocks, nch2), 32 * kGradWarpsPerBlock, 0, fork ? c->side : c->stream>>>(
-            c->T, c->d_gc.p, s.n, s.d_xyz.p, gcoef, mcoef, s.d_tileBox.p, c->d_faceGroup.p, c->d_groups.p, c->fdir,
-            tau, c->d_gradFacets.p, c->nGradFacets, tpc2, grpSta, grpTile,
+        const cudaStream_t st = fork ? c->side : c->stream;
+        const int adjGroups = c->partitioned ? 1 : c->G;
+        float *adjG = c->d_adj32.p, *adjT = adjG + (size_t)adjGroups * s.n;  // reserved by far_workspace
+        k_far_adjoints<<<dim3(cdiv(s.n, 256), adjGroups), 256, 0, st>>>(
+            s.n, adjGroups, c->partitioned ? c->d_staGroup.p : nullptr, c->d_groups.p, gcoef, mcoef, adjG, adjT);
+        c->counters.launches++;
+        const auto far32 = tau >= 3.0 ? k_gradient_warp_far32<true> : k_gradient_warp_far32<false>;
+        far32<<<dim3(fblocks, nch2), 32 * kGradWarpsPerBlock, 0, st>>>(
+            c->T, c->d_gc.p, s.n, s.d_xyz.p, gcoef ? adjG : nullptr, mcoef ? adjT : nullptr, s.d_tileBox.p,
+            c->d_faceGroup.p, c->d_groups.p, c->fdir, tau, c->d_gradFacets.p, c->nGradFacets, tpc2, grpSta, grpTile,
             c->d_partGrad.p + (size_t)(slot0 + nch) * 9 * c->T);
         prof_end(c, c->evGrad, ev2);
         if (fork) {  // join: the main stream waits for the far-field kernel
@@ -1756,6 +1772,7 @@ static lf_status gradient_all(lf_ctx* c, const double* d_params, double* d_grad)
         LF_TRY_CUDA(c, cudaMemsetAsync(c->d_vgrad.p, 0, sizeof(double) * 3 * c->V, c->stream));
     } else {
         LF_TRY_CUDA(c, c->d_partGrad.reserve((size_t)slots * 9 * c->T));
+        LF_RET_IF(far_workspace(c, std::max(gOn ? c->grav.n : 0, mOn ? c->mag.n : 0)));
         int used = 0;
         if (c->sameStations && gOn) {
             used += gradient_set(c, c->grav, c->grav.d_coef.p, mOn ? c->mag.d_coef.p : nullptr, used);
@@ -2266,6 +2283,7 @@ static lf_status jtw_product(lf_ctx* c, StationSet& s, bool grav, const std::vec
                                                              c->d_groups.p, c->d_faceNeeds.p, 1, 1, c->fdir,
                                                              c->d_gc.p);
     LF_TRY_CUDA(c, c->d_partGrad.reserve((size_t)std::max(grad_slots(c, s.n), 1) * 9 * c->T));
+    LF_RET_IF(far_workspace(c, s.n));
     const int used = gradient_set(c, s, grav ? c->d_tmpS.p : nullptr, grav ? nullptr : c->d_tmpS.p, 0);
     if (used > 0 && c->nGradVerts > 0)
         k_vertex_reduce<<<cdiv(c->nGradVerts, 4), 128, 0, c->stream>>>(c->nGradVerts, c->d_gradVerts.p, c->d_vfOff.p,

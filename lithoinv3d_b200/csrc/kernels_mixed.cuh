@@ -178,6 +178,14 @@ __device__ __forceinline__ void pair_near_f64(const double* __restrict__ s, int 
 #undef M
 }
 
+// Paired FP32 (two independent results per instruction, sm_100): each half is
+// rounded as the scalar operation.
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+
 // ---------------------------------------------------- far-field gradient --
 // Sums v[0..31] over the warp, transposed: on return lane L holds the warp
 // total of v[L] in v[0] (31 shuffles for 32 sums instead of 32 x 5).
@@ -208,59 +216,88 @@ __device__ __forceinline__ int tile_gradient_class(const FarKey& k, const double
     return dd >= __dmul_rn(16.0, k.th2) ? 2 : (dd >= k.th2 ? 1 : 0);
 }
 
-constexpr int kFarTerms = 23;      // far-field station sums per facet (listed below)
 constexpr int kFarFlushTiles = 4;  // far tiles summed per lane in FP32 between warp reductions
+
+// FP32 adjoints of the far-field gradient: adjoint x group scale, rounded once
+// per (group, station) instead of once per pair.  Layout [G][S] (G = 1 with
+// every station scaled by its own body's group when sta_group is given).
+__global__ void k_far_adjoints(int S, int G, const int32_t* __restrict__ sta_group,
+                               const GroupConst* __restrict__ groups, const double* __restrict__ gcoef,
+                               const double* __restrict__ mcoef, float* __restrict__ adj_g,
+                               float* __restrict__ adj_t) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= S) return;
+    const int g = sta_group ? sta_group[s] : (int)blockIdx.y;
+    const size_t out = sta_group ? (size_t)s : (size_t)g * S + s;
+    // the scales of k_face_prep_grad (GC_GS, GC_MS)
+    if (gcoef) adj_g[out] = (float)(gcoef[s] * groups[g].gscale_jac);
+    if (mcoef) adj_t[out] = (float)(mcoef[s] * (groups[g].mag_active ? -groups[g].mscale : 0.0));
+}
 
 // Far-field objective gradient in FP32: one warp per facet, lanes over the
 // stations of the facet's far tiles (exactly the tiles k_gradient_warp_fp64
 // leaves out: both classify with facet_far_key / tile_far).  gz by Dunavant's
-// 6-point rule, the 3-point rule beyond 4 tau x size (tile_gradient_class);
-// the point sums are flushed whenever the rule changes.
+// 6-point rule, the 3-point rule beyond 4 tau x size (tile_gradient_class).
 //  * gz: I = A sum_q w_q / r_q, so
 //      sum_s G0 dI/dv = (dA/dv) Q0 - A sum_q beta_qv D_q,
 //    Q0 = sum_s G0 sum_q w_q / r_q, D_q = sum_s G0 w_q (p_q - o) / r_q^3
 //    (G0 = gravity adjoint x group scale, beta_qv = barycentric weight of
 //    point q on vertex v; n_z enters at the end, its own derivative through
 //    the shared finalisation);
-//  * TMI: the closed-form d Omega / dv and d Lambda / dv of the FP64 kernel.
-// Each lane sums up to kFarFlushTiles tiles (8 stations) in FP32; the 23
+//  * TMI: the closed-form d Omega / dv and d Lambda / dv of the FP64 kernel,
+//    in its per-edge form (pair_gradient_fp64).
+// Each lane sums up to kFarFlushTiles tiles (8 stations) in FP32; the 32
 // sums are then reduced across the warp in one transposed pass and lane k
-// adds sum k to its FP64 total.  Lane 0 gathers the totals, forms the facet
-// accumulators in FP64 and finalises.  Facet list and station chunks as in
-// k_gradient_warp_fp64; part layout [chunk][9][T].
-// Sums: 0 Q0; 1-3, 4-6, 7-9 sum_q beta_q{a,b,c} D_q; 10-12, 13-15, 16-18 TMI
-// vertex terms of a, b, c; 19 sum Ts Omega; 20-22 sum Ts Lambda_i.
-// Four CTAs per SM (at most 128 registers, a few bytes of spill) ran faster
-// than the unconstrained 147-register, three-CTA build on every workload
-// measured (contact model -1 %, large model -3 %, 256-body batch -7 %).
-__global__ void __launch_bounds__(128, 4) k_gradient_warp_far32(int T, const double* __restrict__ gc, int S,
-                                                             const double* __restrict__ sta,
-                                                             const double* __restrict__ gcoef,
-                                                             const double* __restrict__ mcoef,
-                                                             const double* __restrict__ tile_box,
-                                                             const int16_t* __restrict__ face_group,
-                                                             const GroupConst* __restrict__ groups, d3 fdir,
-                                                             double tau, const int32_t* __restrict__ facets, int nfacets,
-        int tiles_per_chunk, const int32_t* __restrict__ grp_sta_off,
-        const int32_t* __restrict__ grp_tile_off, double* __restrict__ part) {
+// adds sum k to its FP64 total (one per quadrature rule).  Lane 0 gathers the
+// totals, forms the facet accumulators in FP64 and finalises.  Facet list and
+// station chunks as in k_gradient_warp_fp64; part layout [chunk][9][T].
+// Sums: 0-5, 6-11, 12-17 x, y, z of D_q; 18 Q0; 19-21, 22-24, 25-27 TMI vertex
+// terms of a, b, c; 28 sum Ts Omega / 2; 29-31 sum Ts Lambda_i / 2.
+// SHORT (tau >= 3): pair_far_f32's bounds on e and t hold, so that the series
+// need no fall-back to library functions: through the seventh power beyond
+// 4 tau x size (the omitted terms are below 2e-12), through the ninth nearer,
+// and through the thirteenth for the few pairs with an e above 0.2.
+//
+// Bound by instruction issue.  The quadrature points, the series (three atanh
+// and one atan) and edges 1 and 2 run in pairs through the sm_100 paired FP32
+// instructions; pairing within one (station, facet) needs no more registers
+// than the scalar form, where pairing two stations does.  The vertex sums keep
+// the scalar form's order of additions.  With the adjoints rounded once per
+// station, no range test with library fall-backs and no branch on a
+// lane's adjoints: 264 warp instructions per 32 pairs instead of about 390,
+// both gradient kernels of a 32-body batch (1.29e9 pairs) 18.3 -> 14.6 ms.
+// Four CTAs per SM (128 registers, some spill): three without spill 5 %
+// slower, five 5 %; the facet frame or points in shared memory instead of
+// registers 2 %; the flush through shared memory instead of shuffles equal.
+template <bool SHORT>
+__global__ void __launch_bounds__(128, 4) k_gradient_warp_far32(
+    int T, const double* __restrict__ gc, int S, const double* __restrict__ sta, const float* __restrict__ adj_g,
+    const float* __restrict__ adj_t, const double* __restrict__ tile_box, const int16_t* __restrict__ face_group,
+    const GroupConst* __restrict__ groups, d3 fdir, double tau, const int32_t* __restrict__ facets, int nfacets,
+    int tiles_per_chunk, const int32_t* __restrict__ grp_sta_off, const int32_t* __restrict__ grp_tile_off,
+    double* __restrict__ part) {
     const int lane = threadIdx.x & 31;
     const int w = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
     if (w >= nfacets) return;  // warp-uniform
-    const int f = facets[w];
+    const int f = facets[w], grp = face_group[f];
     if (grp_sta_off) {  // batched bodies: only the facet's own body's stations
-        const int g = face_group[f], sb = grp_sta_off[g];
-        S = grp_sta_off[g + 1] - sb;
+        const int sb = grp_sta_off[grp];
+        S = grp_sta_off[grp + 1] - sb;
         sta += 3 * (size_t)sb;
-        if (gcoef) gcoef += sb;
-        if (mcoef) mcoef += sb;
-        tile_box += 6 * (size_t)grp_tile_off[g];
+        if (adj_g) adj_g += sb;
+        if (adj_t) adj_t += sb;
+        tile_box += 6 * (size_t)grp_tile_off[grp];
+    } else {
+        if (adj_g) adj_g += (size_t)grp * S;
+        if (adj_t) adj_t += (size_t)grp * S;
     }
     // this chunk's station tiles
     const int ntiles_all = (S + kStationTile - 1) / kStationTile;
     const int tbeg = blockIdx.y * tiles_per_chunk, ntiles = min(ntiles_all, tbeg + tiles_per_chunk);
     part += (size_t)blockIdx.y * 9 * T;
+    __shared__ double totals[4][2][32];  // per warp: six-point rule, three-point rule
     bool active, any = false;
-    double tot = 0.0;
+    double tot = 0.0, tot3 = 0.0;
     {
         double C[NGC];
 #pragma unroll
@@ -268,57 +305,47 @@ __global__ void __launch_bounds__(128, 4) k_gradient_warp_far32(int T, const dou
         active = facet_grad_active(C);
         if (active) {
             const float L0 = (float)C[GC_L0], cx = (float)C[GC_CX], cy = (float)C[GC_CY];
-            const float e1x = (float)C[GC_E1X], e1y = (float)C[GC_E1Y], L1 = (float)C[GC_L1];
-            const float e2x = (float)C[GC_E2X], e2y = (float)C[GC_E2Y], L2 = (float)C[GC_L2];
+            const float L1 = (float)C[GC_L1], L2 = (float)C[GC_L2];
+            const float2 ex = make_float2((float)C[GC_E1X], (float)C[GC_E2X]),  // edges 1 and 2
+                         ey = make_float2((float)C[GC_E1Y], (float)C[GC_E2Y]);
             const float rx0 = (float)C[GC_XX], rx1 = (float)C[GC_XY], rx2 = (float)C[GC_XZ];
             const float ry0 = (float)C[GC_YX], ry1 = (float)C[GC_YY], ry2 = (float)C[GC_YZ];
-            const float mf = (float)C[GC_MF], mt0 = (float)C[GC_MT0], mt1 = (float)C[GC_MT1],
-                        mt2 = (float)C[GC_MT2];
+            const float mf = (float)C[GC_MF], mt0 = (float)C[GC_MT0];
+            const float2 mt = make_float2((float)C[GC_MT1], (float)C[GC_MT2]);
             const float A2 = L0 * cy;
             const double ax = C[GC_AX], ay = C[GC_AY], az = C[GC_AZ];
             const double zx = C[GC_ZX], zy = C[GC_ZY], zz = C[GC_ZZ];
-            const double gsn = C[GC_GS], ms = C[GC_MS];
-            float qx[6], qy[6];
+            float2 qx[3], qy[3];  // points 2p, 2p + 1
 #pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                qx[q] = kDun6Bb[q] * L0 + kDun6Bc[q] * cx;
-                qy[q] = kDun6Bc[q] * cy;
+            for (int p = 0; p < 3; ++p) {
+                qx[p] = make_float2(kDun6Bb[2 * p] * L0 + kDun6Bc[2 * p] * cx,
+                                    kDun6Bb[2 * p + 1] * L0 + kDun6Bc[2 * p + 1] * cx);
+                qy[p] = make_float2(kDun6Bc[2 * p] * cy, kDun6Bc[2 * p + 1] * cy);
             }
-            float q0 = 0.f, dqx[6], dqy[6], dqz[6];
-            float vax = 0.f, vay = 0.f, vaz = 0.f, vbx = 0.f, vby = 0.f, vbz = 0.f, vcx = 0.f, vcy = 0.f, vcz = 0.f;
-            float amf = 0.f, amt0 = 0.f, amt1 = 0.f, amt2 = 0.f;
+            const float2 zero = make_float2(0.f, 0.f);
+            float q0 = 0.f;
+            float2 dqx[3], dqy[3], dqz[3];
+            // (b, c) from the first corners of edges 1 and 2, (c, a) from their second corners
+            float2 bcx = zero, bcy = zero, bcz = zero, cax = zero, cay = zero, caz = zero;
+            float2 am01 = zero, am2f = zero;  // sums of Ts Lambda_{0,1} / 2; Ts Lambda_2 / 2, Ts Omega / 2
 #pragma unroll
-            for (int q = 0; q < 6; ++q) dqx[q] = dqy[q] = dqz[q] = 0.f;
+            for (int p = 0; p < 3; ++p) dqx[p] = dqy[p] = dqz[p] = zero;
             int pending = 0, rule = 0;  // rule of the pending point sums: 0 six-point, 1 three-point
             auto flush = [&]() {
-                float v[32];
-                float sa0 = 0.f, sa1 = 0.f, sa2 = 0.f, sb0 = 0.f, sb1 = 0.f, sb2 = 0.f, sc0 = 0.f, sc1 = 0.f, sc2 = 0.f;
-#pragma unroll
-                for (int q = 0; q < 6; ++q) {
-                    // slots 0-2 hold the three-point rule's sums when rule == 1 (slots 3-5 are then zero)
-                    const float bb = rule ? (q < 3 ? kTri3Bb[q] : 0.f) : kDun6Bb[q];
-                    const float bc = rule ? (q < 3 ? kTri3Bc[q] : 0.f) : kDun6Bc[q];
-                    const float ba = 1.f - bb - bc;
-                    sa0 = fmaf(ba, dqx[q], sa0); sa1 = fmaf(ba, dqy[q], sa1); sa2 = fmaf(ba, dqz[q], sa2);
-                    sb0 = fmaf(bb, dqx[q], sb0); sb1 = fmaf(bb, dqy[q], sb1); sb2 = fmaf(bb, dqz[q], sb2);
-                    sc0 = fmaf(bc, dqx[q], sc0); sc1 = fmaf(bc, dqy[q], sc1); sc2 = fmaf(bc, dqz[q], sc2);
-                    dqx[q] = dqy[q] = dqz[q] = 0.f;
-                }
-                v[0] = q0;
-                v[1] = sa0; v[2] = sa1; v[3] = sa2;
-                v[4] = sb0; v[5] = sb1; v[6] = sb2;
-                v[7] = sc0; v[8] = sc1; v[9] = sc2;
-                v[10] = vax; v[11] = vay; v[12] = vaz;
-                v[13] = vbx; v[14] = vby; v[15] = vbz;
-                v[16] = vcx; v[17] = vcy; v[18] = vcz;
-                v[19] = amf; v[20] = amt0; v[21] = amt1; v[22] = amt2;
-#pragma unroll
-                for (int k = kFarTerms; k < 32; ++k) v[k] = 0.f;
-                tot += (double)warp_transpose_sum32(v);
+                float v[32] = {dqx[0].x, dqx[0].y, dqx[1].x, dqx[1].y, dqx[2].x, dqx[2].y,
+                               dqy[0].x, dqy[0].y, dqy[1].x, dqy[1].y, dqy[2].x, dqy[2].y,
+                               dqz[0].x, dqz[0].y, dqz[1].x, dqz[1].y, dqz[2].x, dqz[2].y,
+                               q0, cax.y, cay.y, caz.y, bcx.x, bcy.x, bcz.x,
+                               bcx.y + cax.x, bcy.y + cay.x, bcz.y + caz.x, am2f.y, am01.x, am01.y, am2f.x};
+                const double sum = (double)warp_transpose_sum32(v);
+                if (rule) tot3 += sum;
+                else tot += sum;
                 q0 = 0.f;
-                vax = vay = vaz = vbx = vby = vbz = vcx = vcy = vcz = 0.f;
-                amf = amt0 = amt1 = amt2 = 0.f;
+                bcx = bcy = bcz = cax = cay = caz = am01 = am2f = zero;
+#pragma unroll
+                for (int p = 0; p < 3; ++p) dqx[p] = dqy[p] = dqz[p] = zero;
             };
+            const bool doG = adj_g && C[GC_GS] != 0.0, doT = adj_t && C[GC_MS] != 0.0;
             const FarKey key = facet_far_key(C, tau);
             for (int t0 = tbeg; t0 < ntiles; t0 += 32) {
                 const int t = t0 + lane;
@@ -335,108 +362,129 @@ __global__ void __launch_bounds__(128, 4) k_gradient_warp_far32(int T, const dou
                         pending = 0;
                     }
                     rule = r;
+                    const bool brief = SHORT && r;
                     const int s0 = (t0 + b) * kStationTile;
 #pragma unroll
                     for (int k = 0; k < kStationTile; k += 32) {
-                        const int j = s0 + k + lane;
-                        float G0 = 0.f, Ts = 0.f;
-                        double ox = 0.0, oy = 0.0, oz = 0.0;
-                        if (j < S) {
-                            G0 = (float)((gcoef ? gcoef[j] : 0.0) * gsn);
-                            Ts = (float)((mcoef ? mcoef[j] : 0.0) * ms);
-                            ox = sta[3 * j]; oy = sta[3 * j + 1]; oz = sta[3 * j + 2];
-                        }
-                        if (G0 == 0.f && Ts == 0.f) continue;
+                        // lanes past the last station repeat it with zero adjoints
+                        const int j = min(s0 + k + lane, S - 1);
+                        const bool in = s0 + k + lane < S;
+                        const float G0 = doG && in ? adj_g[j] : 0.f, Ts = doT && in ? adj_t[j] : 0.f;
+                        const double ox = sta[3 * j], oy = sta[3 * j + 1], oz = sta[3 * j + 2];
                         const double ddx = ox - ax, ddy = oy - ay, ddz = oz - az;
                         const float dx = (float)ddx, dy = (float)ddy, dzf = (float)ddz;
                         const float x = fmaf(dx, rx0, fmaf(dy, rx1, dzf * rx2));
                         const float y = fmaf(dx, ry0, fmaf(dy, ry1, dzf * ry2));
                         const float z = (float)(ddx * zx + ddy * zy + ddz * zz);
                         const float z2 = z * z;
-                        if (G0 != 0.f && r) {  // beyond 4 tau: the 3-point rule, weights 1/3
+                        const float2 zz2 = dup2(z2), nx = dup2(-x), ny = dup2(-y), nz = dup2(-z);
+                        if (doG && r) {  // beyond 4 tau: the 3-point rule, weights 1/3
+                            // points 0 and 1 paired, point 2 alone
+                            const float2 px = fma2(make_float2(kTri3Bb[0], kTri3Bb[1]), dup2(L0),
+                                                   fma2(make_float2(kTri3Bc[0], kTri3Bc[1]), dup2(cx), nx));
+                            const float2 py = fma2(make_float2(kTri3Bc[0], kTri3Bc[1]), dup2(cy), ny);
+                            const float2 r2 = fma2(px, px, fma2(py, py, zz2));
+                            const float2 rs = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+                            const float2 g3 = mul2(mul2(mul2(dup2(G0), mul2(dup2(1.f / 3.f), rs)), rs), rs);
+                            dqx[0] = fma2(g3, px, dqx[0]);
+                            dqy[0] = fma2(g3, py, dqy[0]);
+                            dqz[0] = fma2(g3, nz, dqz[0]);
+                            const float px2 = fmaf(kTri3Bb[2], L0, fmaf(kTri3Bc[2], cx, -x));
+                            const float py2 = fmaf(kTri3Bc[2], cy, -y);
+                            const float rs2 = rsqrtf(fmaf(px2, px2, fmaf(py2, py2, z2)));
+                            const float h3 = G0 * ((1.f / 3.f) * rs2) * rs2 * rs2;
+                            dqx[1].x = fmaf(h3, px2, dqx[1].x);
+                            dqy[1].x = fmaf(h3, py2, dqy[1].x);
+                            dqz[1].x = fmaf(h3, -z, dqz[1].x);
+                            q0 = fmaf(G0, fmaf(1.f / 3.f, rs2, fmaf(1.f / 3.f, rs.y, (1.f / 3.f) * rs.x)), q0);
+                        } else if (doG) {
                             float sw = 0.f;
 #pragma unroll
-                            for (int q = 0; q < 3; ++q) {
-                                const float px = fmaf(kTri3Bb[q], L0, fmaf(kTri3Bc[q], cx, -x));
-                                const float py = fmaf(kTri3Bc[q], cy, -y);
-                                const float rs = rsqrtf(fmaf(px, px, fmaf(py, py, z2)));
-                                const float w = (1.f / 3.f) * rs;
-                                sw += w;
-                                const float g3 = G0 * w * rs * rs;
-                                dqx[q] = fmaf(g3, px, dqx[q]);
-                                dqy[q] = fmaf(g3, py, dqy[q]);
-                                dqz[q] = fmaf(g3, -z, dqz[q]);
-                            }
-                            q0 = fmaf(G0, sw, q0);
-                        } else if (G0 != 0.f) {
-                            float sw = 0.f;
-#pragma unroll
-                            for (int q = 0; q < 6; ++q) {
-                                const float px = qx[q] - x, py = qy[q] - y;
-                                const float rs = rsqrtf(fmaf(px, px, fmaf(py, py, z2)));
-                                const float w = kDun6W[q] * rs;
-                                sw += w;
-                                const float g3 = G0 * w * rs * rs;
-                                dqx[q] = fmaf(g3, px, dqx[q]);
-                                dqy[q] = fmaf(g3, py, dqy[q]);
-                                dqz[q] = fmaf(g3, -z, dqz[q]);
+                            for (int p = 0; p < 3; ++p) {
+                                const float2 px = add2(qx[p], nx), py = add2(qy[p], ny);
+                                const float2 r2 = fma2(px, px, fma2(py, py, zz2));
+                                const float2 rs = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+                                const float2 w = mul2(make_float2(kDun6W[2 * p], kDun6W[2 * p + 1]), rs);
+                                sw = fmaf(kDun6W[2 * p], rs.x, sw);
+                                sw = fmaf(kDun6W[2 * p + 1], rs.y, sw);
+                                const float2 g3 = mul2(mul2(mul2(dup2(G0), w), rs), rs);
+                                dqx[p] = fma2(g3, px, dqx[p]);
+                                dqy[p] = fma2(g3, py, dqy[p]);
+                                dqz[p] = fma2(g3, nz, dqz[p]);
                             }
                             q0 = fmaf(G0, sw, q0);
                         }
-                        if (Ts != 0.f) {
-                            const float rbx = L0 - x, rcx = cx - x, rcy = cy - y;
-                            const float la = sqrt_pos(fmaf(x, x, fmaf(y, y, z2)));
-                            const float lb = sqrt_pos(fmaf(rbx, rbx, fmaf(y, y, z2)));
-                            const float lc = sqrt_pos(fmaf(rcx, rcx, fmaf(rcy, rcy, z2)));
-                            const float dab = fmaf(-x, rbx, fmaf(y, y, z2));
-                            const float dac = fmaf(-x, rcx, fmaf(-y, rcy, z2));
-                            const float dbc = fmaf(rbx, rcx, fmaf(-y, rcy, z2));
-                            const float den = la * lb * lc + dab * lc + dac * lb + dbc * la;
-                            const float ny = -z * A2;
-                            const float e0 = __fdividef(L0, la + lb), e1 = __fdividef(L1, lb + lc),
-                                        e2 = __fdividef(L2, lc + la);
-                            float om, l0, l1, l2;
-                            if (far_series_ok(ny, den, e0, e1, e2)) {
-                                om = 2.f * atan_series(__fdividef(ny, den));
-                                l0 = 2.f * atanh_series(e0);
-                                l1 = 2.f * atanh_series(e1);
-                                l2 = 2.f * atanh_series(e2);
-                            } else {
-                                om = 2.f * atan2_far(ny, den);
-                                l0 = lam_f32(la, lb, L0);
-                                l1 = lam_f32(lb, lc, L1);
-                                l2 = lam_f32(lc, la, L2);
-                            }
-                            const float s11 = fmaf(rbx, e1x, -y * e1y), s21 = fmaf(rcx, e2x, rcy * e2y);
+                        if (doT) {
+                            const float2 rx = add2(make_float2(L0, cx), nx);   // b, c
+                            const float2 ry = make_float2(-y, cy - y);         // b, c
+                            const float2 yz = fma2(ry, ry, zz2);
+                            const float2 bc2 = fma2(rx, rx, yz);
+                            const float la2 = fmaf(x, x, yz.x);
+                            const float la = sqrt_pos(la2);
+                            const float2 lbc = mul2(bc2, make_float2(rsqrtf(bc2.x), rsqrtf(bc2.y)));
+                            const float lb = lbc.x, lc = lbc.y;
                             const float ia = __fdividef(1.f, la), ib = __fdividef(1.f, lb), ic = __fdividef(1.f, lc);
+                            const float2 ibc = make_float2(ib, ic), ica = make_float2(ic, ia);
+                            const float u = fmaf(ry.x, ry.y, z2);
+                            const float2 dad = fma2(nx, rx, make_float2(yz.x, u));  // ra.rb, ra.rc
+                            const float dab = dad.x, dac = dad.y, dbc = fmaf(rx.x, rx.y, u);
+                            const float den = fmaf(dbc, la, fmaf(dac, lb, fmaf(dab, lc, la * lb * lc)));
+                            const float nyv = -z * A2;
+                            const float t = __fdividef(nyv, den);
+                            const float2 ea = make_float2(__fdividef(L0, la + lb), __fdividef(L1, lb + lc)),
+                                         eb = make_float2(__fdividef(L2, lc + la), t);
+                            float2 la01, la2f;  // (Lambda_0, Lambda_1) / 2, (Lambda_2, Omega) / 2
+                            const float2 wa = mul2(ea, ea), wb = mul2(eb, eb);
+                            const float2 s3 = make_float2(1.f / 3.f, -1.f / 3.f), s7 = make_float2(1.f / 7.f, -1.f / 7.f);
+                            if (brief) {  // through e^7 and t^7; e < 0.045, |t| < 0.002
+                                la01 = fma2(wa, fma2(wa, dup2(1.f / 7.f), dup2(0.2f)), dup2(1.f / 3.f));
+                                la2f = fma2(wb, fma2(wb, s7, dup2(0.2f)), s3);
+                            } else {
+                                la01 = fma2(wa, fma2(wa, fma2(wa, dup2(1.f / 9.f), dup2(1.f / 7.f)), dup2(0.2f)), dup2(1.f / 3.f));
+                                la2f = fma2(wb, fma2(wb, fma2(wb, dup2(1.f / 9.f), s7), dup2(0.2f)), s3);
+                            }
+                            if (SHORT && !brief && fmaxf(ea.x, fmaxf(ea.y, eb.x)) > 0.2f) {  // e < 0.215: through e^13
+                                const float2 c = make_float2(1.f / 11.f, 1.f / 13.f);
+                                la01 = fma2(wa, fma2(wa, fma2(wa, fma2(wa, fma2(wa, dup2(c.y), dup2(c.x)), dup2(1.f / 9.f)),
+                                                              dup2(1.f / 7.f)), dup2(0.2f)), dup2(1.f / 3.f));
+                                la2f.x = fmaf(wb.x, fmaf(wb.x, fmaf(wb.x, fmaf(wb.x, fmaf(wb.x, c.y, c.x), 1.f / 9.f),
+                                                                    1.f / 7.f), 0.2f), 1.f / 3.f);
+                            }
+                            la01 = mul2(ea, fma2(wa, la01, dup2(1.f)));
+                            la2f = mul2(eb, fma2(wb, la2f, dup2(1.f)));
+                            if (!SHORT && !far_series_ok(nyv, den, ea.x, ea.y, eb.x)) {
+                                la01 = make_float2(0.5f * lam_f32(la, lb, L0), 0.5f * lam_f32(lb, lc, L1));
+                                la2f = make_float2(0.5f * lam_f32(lc, la, L2), atan2_far(nyv, den));
+                            }
+                            am01 = fma2(dup2(Ts), la01, am01);
+                            am2f = fma2(dup2(Ts), la2f, am2f);
                             const float kom = Ts * mf;
                             // edge (p1 -> p2): W = L / (d1 d2 + r1.r2), q = r1 - s1 e, Z = e x r1,
-                            // P = W (kom Z - kl q); p1 += (P - kl e)/d1, p2 += (P + kl e)/d2
-                            auto edge = [&](float r1x, float r1y, float r2x, float r2y, float d1, float d2, float ex,
-                                            float ey, float L, float s1, float kl, float i1, float i2, float& g1x,
-                                            float& g1y, float& g1z, float& g2x, float& g2y, float& g2z) {
-                                const float W = __fdividef(L, fmaf(d1, d2, fmaf(r1x, r2x, fmaf(r1y, r2y, z2))));
-                                const float qxv = fmaf(-s1, ex, r1x), qyv = fmaf(-s1, ey, r1y), qzv = -z;
-                                const float Zx = -ey * z, Zy = ex * z, Zz = fmaf(ex, r1y, -ey * r1x);  // e x r1
-                                const float Px = W * fmaf(kom, Zx, -kl * qxv), Py = W * fmaf(kom, Zy, -kl * qyv),
-                                            Pz = W * fmaf(kom, Zz, -kl * qzv);
-                                g1x = fmaf(fmaf(-kl, ex, Px), i1, g1x);
-                                g1y = fmaf(fmaf(-kl, ey, Py), i1, g1y);
-                                g1z = fmaf(Pz, i1, g1z);
-                                g2x = fmaf(fmaf(kl, ex, Px), i2, g2x);
-                                g2y = fmaf(fmaf(kl, ey, Py), i2, g2y);
-                                g2z = fmaf(Pz, i2, g2z);
-                            };
-                            edge(-x, -y, rbx, -y, la, lb, 1.f, 0.f, L0, -x, Ts * mt0, ia, ib, vax, vay, vaz, vbx, vby,
-                                 vbz);
-                            edge(rbx, -y, rcx, rcy, lb, lc, e1x, e1y, L1, s11, Ts * mt1, ib, ic, vbx, vby, vbz, vcx,
-                                 vcy, vcz);
-                            edge(rcx, rcy, -x, -y, lc, la, e2x, e2y, L2, s21, Ts * mt2, ic, ia, vcx, vcy, vcz, vax,
-                                 vay, vaz);
-                            amf = fmaf(Ts, om, amf);
-                            amt0 = fmaf(Ts, l0, amt0);
-                            amt1 = fmaf(Ts, l1, amt1);
-                            amt2 = fmaf(Ts, l2, amt2);
+                            // P = W (kom Z - kl q); p1 += (P - kl e)/d1, p2 += (P + kl e)/d2.
+                            {  // edge 0: e = (1, 0), so q = (0, -y, -z) and Z = (0, z, -y)
+                                const float kl = Ts * mt0, W = __fdividef(L0, fmaf(la, lb, dab));
+                                const float Py = W * fmaf(kom, z, kl * y), Pz = W * fmaf(kom, -y, kl * z);
+                                cax.y = fmaf(-kl, ia, cax.y);
+                                cay.y = fmaf(Py, ia, cay.y);
+                                caz.y = fmaf(Pz, ia, caz.y);
+                                bcx.x = fmaf(kl, ib, bcx.x);
+                                bcy.x = fmaf(Py, ib, bcy.x);
+                                bcz.x = fmaf(Pz, ib, bcz.x);
+                            }
+                            // edges 1 (b->c) and 2 (c->a), paired
+                            const float2 kl = mul2(dup2(Ts), mt), nkl = neg2(kl), kom2 = dup2(kom);
+                            const float2 W = make_float2(__fdividef(L1, fmaf(lb, lc, dbc)), __fdividef(L2, fmaf(lc, la, dac)));
+                            const float2 ns = neg2(fma2(rx, ex, mul2(ry, ey)));  // -(r1 . e)
+                            const float2 kqx = mul2(nkl, fma2(ns, ex, rx)), kqy = mul2(nkl, fma2(ns, ey, ry));
+                            const float2 Px = mul2(W, fma2(kom2, mul2(ey, nz), kqx)),
+                                         Py = mul2(W, fma2(kom2, mul2(neg2(ex), nz), kqy)),
+                                         Pz = mul2(W, fma2(kom2, fma2(ex, ry, mul2(neg2(ey), rx)), mul2(nkl, nz)));
+                            const float2 t2x=fma2(kl, ex, Px), t2y=fma2(kl, ey, Py);
+                            cax.y = fmaf(t2x.y, ia, cax.y); cay.y = fmaf(t2y.y, ia, cay.y); caz.y = fmaf(Pz.y, ia, caz.y);
+                            bcx.y = fmaf(t2x.x, ic, bcx.y); bcy.y = fmaf(t2y.x, ic, bcy.y); bcz.y = fmaf(Pz.x, ic, bcz.y);
+                            bcx = fma2(fma2(nkl, ex, Px), ibc, bcx);
+                            bcy = fma2(fma2(nkl, ey, Py), ibc, bcy);
+                            bcz = fma2(Pz, ibc, bcz);
                         }
                     }
                     if (++pending == kFarFlushTiles) {
@@ -449,28 +497,40 @@ __global__ void __launch_bounds__(128, 4) k_gradient_warp_far32(int T, const dou
         }
     }
     double outv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (active && any) {
-        double v[kFarTerms];
-#pragma unroll
-        for (int k = 0; k < kFarTerms; ++k) v[k] = __shfl_sync(0xffffffffu, tot, k);
+    if (active && any) {  // warp-uniform
+        double(*v)[32] = totals[threadIdx.x >> 5];
+        v[0][lane] = tot;
+        v[1][lane] = tot3;
+        __syncwarp();
         if (lane == 0) {
             double C[NGC];
 #pragma unroll
             for (int k = 0; k < NGC; ++k) C[k] = __ldcg(&gc[(size_t)k * T + f]);
             const double nz = C[GC_ZZ], L0 = C[GC_L0], cx = C[GC_CX], cy = C[GC_CY];
-            const double Ar = 0.5 * L0 * cy, q0 = v[0];
+            const double Ar = 0.5 * L0 * cy, q0 = v[0][18] + v[1][18];
+            d3 Da = mk3(0, 0, 0), Db = Da, Dc = Da;  // sum_q beta_q{a,b,c} D_q over both rules
+            for (int q = 0; q < 9; ++q) {
+                const int rl = q >= 6, k = rl ? q - 6 : q;
+                const double bb = rl ? kTri3Bb[k] : kDun6Bb[k], bc = rl ? kTri3Bc[k] : kDun6Bc[k];
+                const d3 D = mk3(v[rl][k], v[rl][6 + k], v[rl][12 + k]);
+                Da = Da + D * (1.0 - bb - bc);
+                Db = Db + D * bb;
+                Dc = Dc + D * bc;
+            }
+            auto both = [&](int k) { return v[0][k] + v[1][k]; };
             // dA/da = (-cy, cx - L0, 0)/2, dA/db = (cy, -cx, 0)/2, dA/dc = (0, L0, 0)/2
             GradAcc A;
             grad_acc_zero(A);
-            A.va = mk3(nz * (-0.5 * cy * q0 - Ar * v[1]) + v[10], nz * (0.5 * (cx - L0) * q0 - Ar * v[2]) + v[11],
-                       nz * (-Ar * v[3]) + v[12]);
-            A.vb = mk3(nz * (0.5 * cy * q0 - Ar * v[4]) + v[13], nz * (-0.5 * cx * q0 - Ar * v[5]) + v[14],
-                       nz * (-Ar * v[6]) + v[15]);
-            A.vc = mk3(nz * (-Ar * v[7]) + v[16], nz * (0.5 * L0 * q0 - Ar * v[8]) + v[17], nz * (-Ar * v[9]) + v[18]);
+            A.va = mk3(nz * (-0.5 * cy * q0 - Ar * Da.x) + both(19), nz * (0.5 * (cx - L0) * q0 - Ar * Da.y) + both(20),
+                       nz * (-Ar * Da.z) + both(21));
+            A.vb = mk3(nz * (0.5 * cy * q0 - Ar * Db.x) + both(22), nz * (-0.5 * cx * q0 - Ar * Db.y) + both(23),
+                       nz * (-Ar * Db.z) + both(24));
+            A.vc = mk3(nz * (-Ar * Dc.x) + both(25), nz * (0.5 * L0 * q0 - Ar * Dc.y) + both(26),
+                       nz * (-Ar * Dc.z) + both(27));
             A.ai = Ar * q0;
-            A.amf = v[19];
-            A.amt[0] = v[20]; A.amt[1] = v[21]; A.amt[2] = v[22];
-            grad_finalize(C, A, groups[face_group[f]], fdir, outv);
+            A.amf = 2.0 * both(28);
+            for (int i = 0; i < 3; ++i) A.amt[i] = 2.0 * both(29 + i);
+            grad_finalize(C, A, groups[grp], fdir, outv);
         }
     }
     if (lane == 0)
