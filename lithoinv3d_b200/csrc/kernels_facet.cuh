@@ -22,8 +22,8 @@ struct __align__(16) FaceF32 {
     float ry0, ry1, ry2, cx;   // local y axis, c.x
     float cy, L1, L2, gq;      // c.y, |bc|, |ca|, n_z * gz scale * area
     float mf, mt0, mt1, mt2;   // TMI facet scales, doubled
-    float q6[12];              // (x, y) of the 6-point rule's points in the local frame
-    float q3[8];               // (x, y) of the 3-point rule's points, pad
+    float q6[12];              // 6-point rule in the local frame: x, x, y, y of two points at a time
+    float q3[8];               // 3-point rule: x, x, y, y of two points, x, y of the third, pad
     double ax, ay, az, zx, zy, zz;
     float cenx, ceny, cenz;    // centroid
     float size;                // longest edge; -1 for a facet that contributes nothing
@@ -46,13 +46,15 @@ __device__ __forceinline__ void make_face_f32(const double* m, FaceF32& F) {
     F.mt1 = 2.f * (float)M(MC_MT1); F.mt2 = 2.f * (float)M(MC_MT2);
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-        F.q6[2 * q] = kDun6Bb[q] * F.L0 + kDun6Bc[q] * F.cx;
-        F.q6[2 * q + 1] = kDun6Bc[q] * F.cy;
+        const int k = 4 * (q / 2) + q % 2;
+        F.q6[k] = kDun6Bb[q] * F.L0 + kDun6Bc[q] * F.cx;
+        F.q6[k + 2] = kDun6Bc[q] * F.cy;
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        F.q3[2 * q] = kTri3Bb[q] * F.L0 + kTri3Bc[q] * F.cx;
-        F.q3[2 * q + 1] = kTri3Bc[q] * F.cy;
+        const int k = q < 2 ? q : 4;
+        F.q3[k] = kTri3Bb[q] * F.L0 + kTri3Bc[q] * F.cx;
+        F.q3[q < 2 ? k + 2 : 5] = kTri3Bc[q] * F.cy;
     }
     F.q3[6] = F.q3[7] = 0.f;
     F.ax = M(MC_AX); F.ay = M(MC_AY); F.az = M(MC_AZ);
@@ -209,47 +211,56 @@ __device__ __forceinline__ void pair_far_f32(const FaceF32* Fp, double ox, doubl
     const float z = (float)(ddx * w1.y + ddy * w2.x + ddz * w2.y);
     const float L0 = v0.w, cx = v1.w, cy = v2.x, L1 = v2.y, L2 = v2.z, gq = v2.w;
     const float z2 = z * z;
+    const float2 zz = dup2(z2), nx = dup2(-x), nyy = dup2(-y);
     // gz: n_z * gscale * A * sum_q w_q / r_q.  A facet with a horizontal unit
     // normal (n_z == 0 exactly: every vertical face of a voxel-built surface,
     // which z-only vertex moves keep vertical) has gq == 0 and adds exactly
     // zero, as in the reference's n_z * (...) product; its quadrature is
     // skipped.  The facet is the same for every lane, so the branch is
-    // warp-uniform.
-    if (RULE != RULE_MID) {
+    // warp-uniform.  The record holds the points in pairs (x, x, y, y).
+    if (RULE != RULE_MID && gq != 0.f) {
         float acc = 0.f;
-        if (gq == 0.f) {
-        } else if (RULE == RULE_DUN6) {
-            const float4 qa = v[4], qb = v[5], qc = v[6];
-            const float q[12] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w, qc.x, qc.y, qc.z, qc.w};
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                float px = q[2 * k] - x, py = q[2 * k + 1] - y;
-                acc = fmaf(kDun6W[k], rsqrtf(fmaf(px, px, fmaf(py, py, z2))), acc);
-            }
-        } else {
-            const float4 qa = v[7], qb = v[8];
-            const float q[6] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y};
+        auto two = [&](const float4& q) {  // squared distances of two points
+            const float2 px = add2(make_float2(q.x, q.y), nx), py = add2(make_float2(q.z, q.w), nyy);
+            return fma2(px, px, fma2(py, py, zz));
+        };
+        if (RULE == RULE_DUN6) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                float px = q[2 * k] - x, py = q[2 * k + 1] - y;
-                acc += rsqrtf(fmaf(px, px, fmaf(py, py, z2)));
+                const float2 r2 = two(v[4 + k]);
+                acc = fmaf(kDun6W[2 * k], rsqrtf(r2.x), acc);
+                acc = fmaf(kDun6W[2 * k + 1], rsqrtf(r2.y), acc);
             }
+        } else {
+            const float2 r2 = two(v[7]);
+            const float4 q = v[8];
+            const float px = q.x - x, py = q.y - y;
+            acc += rsqrtf(r2.x);
+            acc += rsqrtf(r2.y);
+            acc += rsqrtf(fmaf(px, px, fmaf(py, py, z2)));
             acc *= (1.f / 3.f);
         }
-        if (gq != 0.f) *gz += gq * acc;
+        *gz += gq * acc;
     }
     // TMI: MF * Omega + sum_i MT_i Lambda_i with Omega = 2 atan2(ny, den) and
     // Lambda_i = 2 atanh(e_i); the record holds 2 MF and 2 MT_i, so the terms
     // below are atan2 and atanh.  Scaling by 2 is exact: the bits equal
     // MF * (2 atan2) + MT_i * (2 atanh).
-    float rbx = L0 - x, rcx = cx - x, rcy = cy - y;
-    float la = sqrt_pos(fmaf(x, x, fmaf(y, y, z2)));
-    float lb = sqrt_pos(fmaf(rbx, rbx, fmaf(y, y, z2)));
-    float lc = sqrt_pos(fmaf(rcx, rcx, fmaf(rcy, rcy, z2)));
-    float dab = fmaf(-x, rbx, fmaf(y, y, z2));
-    float dac = fmaf(-x, rcx, fmaf(-y, rcy, z2));
-    float dbc = fmaf(rbx, rcx, fmaf(-y, rcy, z2));
-    float den = la * lb * lc + dab * lc + dac * lb + dbc * la;
+    const float2 rx = add2(make_float2(L0, cx), nx);  // b, c
+    const float rbx = rx.x, rcx = rx.y;
+    const float2 ry = make_float2(-y, cy - y);        // b, c
+    const float2 yz = fma2(ry, ry, zz);
+    const float2 bc2 = fma2(rx, rx, yz);
+    const float la = sqrt_pos(fmaf(x, x, yz.x));
+    const float2 lbc = mul2(bc2, make_float2(rsqrtf(bc2.x), rsqrtf(bc2.y)));
+    const float lb = lbc.x, lc = lbc.y;
+    const float u = fmaf(ry.x, ry.y, z2);
+    const float2 dd = fma2(nx, rx, make_float2(yz.x, u));  // ra.rb, ra.rc
+    const float dbc = fmaf(rbx, rcx, u);
+    // la lb lc + dab lc + dac lb + dbc la, and the TMI sum below, rounded as in
+    // the one-at-a-time form of each class
+    const float den = fmaf(dbc, la, fmaf(dd.y, lb, RULE == RULE_MID ? fmaf(dd.x, lc, la * lb * lc)
+                                                                    : fmaf(la * lb, lc, dd.x * lc)));
     const float l0cy = L0 * cy;
     const float ny = -z * l0cy;
     float om, l0, l1, l2;
@@ -289,7 +300,13 @@ __device__ __forceinline__ void pair_far_f32(const FaceF32* Fp, double ox, doubl
             *gz += v13.w * h;
         }
     } else {
-        const float e0 = __fdividef(L0, la + lb), e1 = __fdividef(L1, lb + lc), e2 = __fdividef(L2, lc + la);
+        const float2 ea = make_float2(__fdividef(L0, la + lb), __fdividef(L1, lb + lc));
+        const float2 eb = make_float2(__fdividef(L2, lc + la), __fdividef(ny, den));  // e2, t
+        // atanh(e) and atan(t) = e p(e^2), t p(t^2), two at a time
+        const float2 wa = mul2(ea, ea), wb = mul2(eb, eb);
+        const float2 s3 = make_float2(1.f / 3.f, -1.f / 3.f);
+        float2 pa, pb;
+        bool series = true;
         if (SHORT && RULE == RULE_TRI3) {
             // Beyond 12 x size every vertex lies beyond 11.3 x size (a vertex
             // is within 2/3 of a median, so within size, of the centroid):
@@ -297,34 +314,36 @@ __device__ __forceinline__ void pair_far_f32(const FaceF32* Fp, double ox, doubl
             // the solid angle, below area / distance^2, under 0.0035 (|t| <
             // 0.002: through t^3 leaves 1e-12); den > 0 and the range test
             // holds there.
-            const float t = __fdividef(ny, den);
-            om = t * fmaf(t * t, -1.f / 3.f, 1.f);
-            l0 = e0 * fmaf(e0 * e0, fmaf(e0 * e0, 0.2f, 1.f / 3.f), 1.f);
-            l1 = e1 * fmaf(e1 * e1, fmaf(e1 * e1, 0.2f, 1.f / 3.f), 1.f);
-            l2 = e2 * fmaf(e2 * e2, fmaf(e2 * e2, 0.2f, 1.f / 3.f), 1.f);
+            pa = fma2(wa, dup2(0.2f), dup2(1.f / 3.f));
+            pb = fma2(wb, make_float2(0.2f, 0.f), s3);
         } else if (SHORT) {
             // Beyond 3 x size every vertex lies beyond 2.33 x size: e_i < 0.215
             // (one term more than atanh_series, through e^11, leaves 8e-10)
             // and |t| < 0.04 (through t^5 leaves 6e-10); the vertices' view
             // angles stay below 25 degrees, so den > 0.
-            const float t = __fdividef(ny, den), t2 = t * t;
-            om = t * fmaf(t2, fmaf(t2, 0.2f, -1.f / 3.f), 1.f);
-            l0 = e0 * fmaf(e0 * e0, atanh_q11(e0 * e0), 1.f);
-            l1 = e1 * fmaf(e1 * e1, atanh_q11(e1 * e1), 1.f);
-            l2 = e2 * fmaf(e2 * e2, atanh_q11(e2 * e2), 1.f);
-        } else if (far_series_ok(ny, den, e0, e1, e2)) {
-            om = atan_series(__fdividef(ny, den));
-            l0 = atanh_series(e0);
-            l1 = atanh_series(e1);
-            l2 = atanh_series(e2);
+            pa = fma2(wa, fma2(wa, fma2(wa, fma2(wa, dup2(1.f / 11.f), dup2(1.f / 9.f)), dup2(1.f / 7.f)), dup2(0.2f)),
+                      dup2(1.f / 3.f));
+            const float q = fmaf(wb.x, fmaf(wb.x, 1.f / 11.f, 1.f / 9.f), 1.f / 7.f);
+            pb = fma2(wb, fma2(wb, make_float2(q, 0.f), dup2(0.2f)), s3);
         } else {
+            pa = fma2(wa, fma2(wa, fma2(wa, dup2(1.f / 9.f), dup2(1.f / 7.f)), dup2(0.2f)), dup2(1.f / 3.f));
+            pb = fma2(wb, fma2(wb, fma2(wb, dup2(1.f / 9.f), make_float2(1.f / 7.f, -1.f / 7.f)), dup2(0.2f)), s3);
+            series = far_series_ok(ny, den, ea.x, ea.y, eb.x);
+        }
+        pa = mul2(ea, fma2(wa, pa, dup2(1.f)));
+        pb = mul2(eb, fma2(wb, pb, dup2(1.f)));
+        l0 = pa.x;
+        l1 = pa.y;
+        l2 = pb.x;
+        om = pb.y;
+        if (!series) {
             om = atan2_far(ny, den);
             l0 = 0.5f * lam_f32(la, lb, L0);
             l1 = 0.5f * lam_f32(lb, lc, L1);
             l2 = 0.5f * lam_f32(lc, la, L2);
         }
     }
-    *tmi += v3.x * om + v3.y * l0 + v3.z * l1 + v3.w * l2;
+    *tmi += fmaf(v3.w, l2, fmaf(v3.z, l1, RULE == RULE_TRI3 ? fmaf(v3.y, l0, v3.x * om) : fmaf(v3.x, om, v3.y * l0)));
 }
 
 
@@ -430,7 +449,7 @@ __device__ __forceinline__ void forward_mixed_block(FaceF32* __restrict__ smf, d
                 __syncwarp();
                 if (act) {
                     double g1 = 0.0, t1 = 0.0;
-                    pair_near_f64(slot, 0, 1, mk3(ox, oy, oz), &g1, &t1);
+                    pair_near_f64(slot, mk3(ox, oy, oz), &g1, &t1);
                     if (GZ) gz += g1;
                     if (TMI) tmi += t1;
                 }
@@ -444,8 +463,14 @@ __device__ __forceinline__ void forward_mixed_block(FaceF32* __restrict__ smf, d
     }
 }
 
+// Issue slots 74 % busy, special-function pipe 70 % (three to six rsqrt, three
+// rsqrt and four reciprocals, four FP64-to-FP32 conversions a pair): 147 warp
+// instructions per 32 pairs with the points, vertices and series in pairs
+// (162 one by one).  19,076 facets x 4,096 stations: 460 us one by one with
+// library near pairs, 424 us now.  Seven CTAs per SM (72 registers): six
+// 434 us, unbounded 429, eight 423.
 template <bool GZ, bool TMI, int FT>
-__global__ void __launch_bounds__(128) k_forward_mixed(int S, const double* __restrict__ sta, int T,
+__global__ void __launch_bounds__(128, 7) k_forward_mixed(int S, const double* __restrict__ sta, int T,
                                                        const double* __restrict__ mc,
                                                        const FaceF32* __restrict__ mf32,
                                                        const int32_t* __restrict__ chunk_begin,
@@ -463,7 +488,7 @@ __global__ void __launch_bounds__(128) k_forward_mixed(int S, const double* __re
 
 // Batched bodies (item list as for k_forward_fp64_items).
 template <bool GZ, bool TMI, int FT>
-__global__ void __launch_bounds__(128) k_forward_mixed_items(const FwdItem* __restrict__ items, int nitems,
+__global__ void __launch_bounds__(128, 7) k_forward_mixed_items(const FwdItem* __restrict__ items, int nitems,
                                                              const double* __restrict__ sta, int T,
                                                              const double* __restrict__ mc,
                                                              const FaceF32* __restrict__ mf32, float tau,

@@ -145,19 +145,14 @@ __device__ __forceinline__ bool far_series_ok(float ny, float den, float v0, flo
 
 // Near pair in FP64, local frame: solidAngle's branch semantics, Lambda in
 // the symmetric form (lambda_sym: the reference's value except exactly on an
-// edge's line beyond its end, where the reference's branch gives 0).  Adds
-// gz and TMI contributions.
-__device__ __forceinline__ void pair_near_f64(const double* __restrict__ s, int j, int stride, d3 o, double* gz,
-                                              double* tmi) {
-#define M(k) s[(k) * stride + j]
-    double dx = o.x - M(MC_AX), dy = o.y - M(MC_AY), dz = o.z - M(MC_AZ);
-    double x = dx * M(MC_XX) + dy * M(MC_XY) + dz * M(MC_XZ);
-    double y = dx * M(MC_YX) + dy * M(MC_YY) + dz * M(MC_YZ);
-    double z = dx * M(MC_ZX) + dy * M(MC_ZY) + dz * M(MC_ZZ);
-    double L0 = M(MC_L0), cx = M(MC_CX), cy = M(MC_CY);
-    double rbx = L0 - x, rcx = cx - x, rcy = cy - y, z2 = z * z;
-    double la = sqrt(x * x + y * y + z2), lb = sqrt(rbx * rbx + y * y + z2), lc = sqrt(rcx * rcx + rcy * rcy + z2);
-    double h = -z;
+// edge's line beyond its end, where the reference's branch gives 0).  Returns
+// the gz and TMI contributions.  s: the facet's constants, (x, y, z) the
+// station in its frame.
+__device__ __noinline__ double2 pair_near_f64_close(const double* __restrict__ s, double x, double y, double z) {
+    const double L0 = s[MC_L0], cx = s[MC_CX], cy = s[MC_CY];
+    const double rbx = L0 - x, rcx = cx - x, rcy = cy - y, z2 = z * z;
+    const double la = sqrt(x * x + y * y + z2), lb = sqrt(rbx * rbx + y * y + z2), lc = sqrt(rcx * rcx + rcy * rcy + z2);
+    const double h = -z;
     double om = 0.0;
     if (!(la < kEps || lb < kEps || lc < kEps)) {
         double den = la * lb * lc + (-x * rbx + y * y + z2) * lc + (-x * rcx - y * rcy + z2) * lb +
@@ -165,17 +160,46 @@ __device__ __forceinline__ void pair_near_f64(const double* __restrict__ s, int 
         om = 2.0 * atan2(h * (L0 * cy), den);
     }
     bool live;
-    double lam0 = (L0 < kEps) ? 0.0 : lambda_sym(la, lb, L0, &live);
-    double e1x = M(MC_E1X), e1y = M(MC_E1Y), e2x = M(MC_E2X), e2y = M(MC_E2Y);
-    double lam1 = (M(MC_L1) < kEps) ? 0.0 : lambda_sym(lb, lc, M(MC_L1), &live);
-    double lam2 = (M(MC_L2) < kEps) ? 0.0 : lambda_sym(lc, la, M(MC_L2), &live);
+    const double lam0 = (L0 < kEps) ? 0.0 : lambda_sym(la, lb, L0, &live);
+    const double e1x = s[MC_E1X], e1y = s[MC_E1Y], e2x = s[MC_E2X], e2y = s[MC_E2Y];
+    const double lam1 = (s[MC_L1] < kEps) ? 0.0 : lambda_sym(lb, lc, s[MC_L1], &live);
+    const double lam2 = (s[MC_L2] < kEps) ? 0.0 : lambda_sym(lc, la, s[MC_L2], &live);
     // d_perp_i = -(r1 . perp_i), perp_i = z x e_i = (-e_y, e_x, 0)
-    double dp0 = y;
-    double dp1 = rbx * e1y + y * e1x;
-    double dp2 = rcx * e2y - rcy * e2x;
-    *gz += M(MC_SGZ) * (dp0 * lam0 + dp1 * lam1 + dp2 * lam2 - h * om);
-    *tmi += M(MC_MF) * om + M(MC_MT0) * lam0 + M(MC_MT1) * lam1 + M(MC_MT2) * lam2;
-#undef M
+    const double dp0 = y, dp1 = rbx * e1y + y * e1x, dp2 = rcx * e2y - rcy * e2x;
+    return make_double2(s[MC_SGZ] * (dp0 * lam0 + dp1 * lam1 + dp2 * lam2 - h * om),
+                        s[MC_MF] * om + s[MC_MT0] * lam0 + s[MC_MT1] * lam1 + s[MC_MT2] * lam2);
+}
+
+// The same, by polynomials where every L / (d1 + d2) is below 1/2 (see
+// pair_forward_fp64); adds the gz and TMI contributions.  About 3 % of the
+// mixed forward's pairs come here, and through the library functions they
+// cost four times a far pair: 19,076 facets x 4,096 stations 441 us with
+// those, 424 us without (13,388 facets x 1,036 and 7,575 stations: 320, 300 us a launch).
+__device__ __forceinline__ void pair_near_f64(const double* __restrict__ s, d3 o, double* gz, double* tmi) {
+    const double dx = o.x - s[MC_AX], dy = o.y - s[MC_AY], dz = o.z - s[MC_AZ];
+    const double x = dx * s[MC_XX] + dy * s[MC_XY] + dz * s[MC_XZ];
+    const double y = dx * s[MC_YX] + dy * s[MC_YY] + dz * s[MC_YZ];
+    const double z = dx * s[MC_ZX] + dy * s[MC_ZY] + dz * s[MC_ZZ];
+    const double L0 = s[MC_L0], cx = s[MC_CX], cy = s[MC_CY], L1 = s[MC_L1], L2 = s[MC_L2];
+    const double rbx = L0 - x, rcx = cx - x, rcy = cy - y;
+    const double z2 = z * z, yz2 = fma(y, y, z2);
+    const double a2 = fma(x, x, yz2), b2 = fma(rbx, rbx, yz2), c2 = fma(rcx, rcx, fma(rcy, rcy, z2));
+    const double la = sqrt_pos64(a2), lb = sqrt_pos64(b2), lc = sqrt_pos64(c2);
+    const double v0 = L0 * rcp_pos64(la + lb), v1 = L1 * rcp_pos64(lb + lc), v2 = L2 * rcp_pos64(lc + la);
+    if (!(max(__double2hiint(v0), max(__double2hiint(v1), __double2hiint(v2))) < 0x3fe00000)) {
+        const double2 r = pair_near_f64_close(s, x, y, z);
+        *gz += r.x;
+        *tmi += r.y;
+        return;
+    }
+    // ra . rb etc. in the facet's frame
+    const double dab = fma(-x, rbx, yz2), u = fma(-y, rcy, z2), dac = fma(-x, rcx, u), dbc = fma(rbx, rcx, u);
+    const double den = fma(la * lb, lc, fma(dab, lc, fma(dac, lb, dbc * la)));
+    const double om = atan_poly64(-z * (L0 * cy) * rcp_pos64(den));
+    const double l0 = atanh_poly64(v0), l1 = atanh_poly64(v1), l2 = atanh_poly64(v2);  // Lambda / 2
+    const double dp1 = fma(rbx, s[MC_E1Y], y * s[MC_E1X]), dp2 = fma(rcx, s[MC_E2Y], -rcy * s[MC_E2X]);
+    *gz += 2.0 * s[MC_SGZ] * fma(y, l0, fma(dp1, l1, fma(dp2, l2, z * om)));
+    *tmi += 2.0 * fma(s[MC_MF], om, fma(s[MC_MT0], l0, fma(s[MC_MT1], l1, s[MC_MT2] * l2)));
 }
 
 // Paired FP32 (two independent results per instruction, sm_100): each half is
@@ -385,18 +409,19 @@ __global__ void __launch_bounds__(128, 4) k_gradient_warp_far32(
                             const float2 py = fma2(make_float2(kTri3Bc[0], kTri3Bc[1]), dup2(cy), ny);
                             const float2 r2 = fma2(px, px, fma2(py, py, zz2));
                             const float2 rs = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                            const float2 g3 = mul2(mul2(mul2(dup2(G0), mul2(dup2(1.f / 3.f), rs)), rs), rs);
+                            const float2 w = mul2(dup2(1.f / 3.f), rs);
+                            const float2 g3 = mul2(mul2(mul2(dup2(G0), w), rs), rs);
                             dqx[0] = fma2(g3, px, dqx[0]);
                             dqy[0] = fma2(g3, py, dqy[0]);
                             dqz[0] = fma2(g3, nz, dqz[0]);
                             const float px2 = fmaf(kTri3Bb[2], L0, fmaf(kTri3Bc[2], cx, -x));
                             const float py2 = fmaf(kTri3Bc[2], cy, -y);
                             const float rs2 = rsqrtf(fmaf(px2, px2, fmaf(py2, py2, z2)));
-                            const float h3 = G0 * ((1.f / 3.f) * rs2) * rs2 * rs2;
+                            const float w2 = __fmul_rn(1.f / 3.f, rs2), h3 = G0 * w2 * rs2 * rs2;
                             dqx[1].x = fmaf(h3, px2, dqx[1].x);
                             dqy[1].x = fmaf(h3, py2, dqy[1].x);
                             dqz[1].x = fmaf(h3, -z, dqz[1].x);
-                            q0 = fmaf(G0, fmaf(1.f / 3.f, rs2, fmaf(1.f / 3.f, rs.y, (1.f / 3.f) * rs.x)), q0);
+                            q0 = fmaf(G0, __fadd_rn(__fadd_rn(w.x, w.y), w2), q0);
                         } else if (doG) {
                             float sw = 0.f;
 #pragma unroll
@@ -405,8 +430,8 @@ __global__ void __launch_bounds__(128, 4) k_gradient_warp_far32(
                                 const float2 r2 = fma2(px, px, fma2(py, py, zz2));
                                 const float2 rs = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
                                 const float2 w = mul2(make_float2(kDun6W[2 * p], kDun6W[2 * p + 1]), rs);
-                                sw = fmaf(kDun6W[2 * p], rs.x, sw);
-                                sw = fmaf(kDun6W[2 * p + 1], rs.y, sw);
+                                sw = __fadd_rn(sw, w.x);
+                                sw = __fadd_rn(sw, w.y);
                                 const float2 g3 = mul2(mul2(mul2(dup2(G0), w), rs), rs);
                                 dqx[p] = fma2(g3, px, dqx[p]);
                                 dqy[p] = fma2(g3, py, dqy[p]);
@@ -428,7 +453,7 @@ __global__ void __launch_bounds__(128, 4) k_gradient_warp_far32(
                             const float u = fmaf(ry.x, ry.y, z2);
                             const float2 dad = fma2(nx, rx, make_float2(yz.x, u));  // ra.rb, ra.rc
                             const float dab = dad.x, dac = dad.y, dbc = fmaf(rx.x, rx.y, u);
-                            const float den = fmaf(dbc, la, fmaf(dac, lb, fmaf(dab, lc, la * lb * lc)));
+                            const float den = fmaf(dbc, la, fmaf(dac, lb, fmaf(la * lb, lc, dab * lc)));
                             const float nyv = -z * A2;
                             const float t = __fdividef(nyv, den);
                             const float2 ea = make_float2(__fdividef(L0, la + lb), __fdividef(L1, lb + lc)),

@@ -542,7 +542,7 @@ __device__ __forceinline__ bool forward_patch_block(PatchSmem<NT>& sm, int s, bo
             if (lane < NMC) slot[lane] = __ldg(mc + (size_t)lane * T + f);
             __syncwarp();
             double g1 = 0.0, t1 = 0.0;
-            pair_near_f64(slot, 0, 1, mk3(ox, oy, oz), &g1, &t1);
+            pair_near_f64(slot, mk3(ox, oy, oz), &g1, &t1);
             if (GZ) gz += g1;
             if (TMI) tmi += t1;
         }
