@@ -194,6 +194,14 @@ struct lf_ctx {
     DevBuf<int32_t> d_labels, d_grpTriOffDev, d_cGroup, d_cCls, d_ptCls;
     DevBuf<unsigned long long> d_clsMask;  // per-point crossing parities (one bit per group)
     DevBuf<double> d_cMid, d_cThick, d_cPar, d_cPar0, d_cFp, d_cFm, d_cGrad, d_cOut, d_pts;
+    // Side-by-side sweep (k_constraint_sweep): which vertices and triangles each
+    // parameter moves, built on first use.  sweepState 0: not built, 1: built,
+    // -1: the model needs the sequential sweep.
+    int sweepState = 0, sweepMaxVerts = 0;
+    std::vector<int32_t> sweepWhole;  // parameters evaluated by whole passes
+    DevBuf<int32_t> d_swList, d_swAvOff, d_swAv, d_swAtOff, d_swSync, d_swPre;
+    DevBuf<int4> d_swAt;
+    DevBuf<double> d_swSrc;
     int nCons = 0;
     double consWeight = 1e6;  // ConstraintHandler's default weight
 
@@ -802,6 +810,7 @@ extern "C" lf_status lf_set_model_tables(lf_ctx* c, int G, const double* density
     c->planEpoch++;
     c->hasModel = true;
     c->gnReady = false;
+    c->sweepState = 0;
     LF_TRY_CUDA(c, cudaStreamSynchronize(c->stream));
     return LF_OK;
 }
@@ -1112,7 +1121,9 @@ static lf_status upload_chunks(lf_ctx* c) {
     return LF_OK;
 }
 
-static lf_status scatter(lf_ctx* c, const double* d_params) {
+// keep_sources: receives the positions after the parameter writes, which the
+// interpolation reads.
+static lf_status scatter(lf_ctx* c, const double* d_params, double* keep_sources = nullptr) {
     if (c->statelessScatter)
         LF_TRY_CUDA(c, cudaMemcpyAsync(c->d_pos.p, c->d_pos0.p, sizeof(double) * 3 * c->V, cudaMemcpyDeviceToDevice,
                                        c->stream));
@@ -1121,6 +1132,9 @@ static lf_status scatter(lf_ctx* c, const double* d_params) {
                                                                   c->d_refAxis.p, c->d_refScale.p, c->d_pos.p);
         c->counters.launches++;
     }
+    if (keep_sources)
+        LF_TRY_CUDA(c, cudaMemcpyAsync(keep_sources, c->d_pos.p, sizeof(double) * 3 * c->V, cudaMemcpyDeviceToDevice,
+                                       c->stream));
     if (c->nInterpRows > 0) {
         k_interpolate<<<cdiv(c->nInterpRows, 256), 256, 0, c->stream>>>(c->nInterpRows, c->d_interpRows.p,
                                                                          c->d_interpOff.p, c->d_interpSrc.p,
@@ -2926,6 +2940,151 @@ extern "C" lf_status lf_constraint_penalty(lf_ctx* c, const double* params, doub
     return LF_OK;
 }
 
+// Vertices and triangles that each parameter moves (k_constraint_sweep), from
+// the scatter's tables.  A parameter that moves more than kSweepMaxVerts
+// vertices (a control point that drives most of a mesh) gets no list and is
+// evaluated by whole passes.  A model whose tables do not meet the sweep's
+// assumptions (a row that reads a row, a vertex in two averaging groups), whose
+// lists are too long, or with more than kSweepMostWhole such parameters keeps
+// the sequential sweep.
+static lf_status sweep_tables(lf_ctx* c) {
+    if (c->sweepState != 0) return LF_OK;
+    const int V = c->V, T = c->T, np = c->np;
+    auto fetch = [&](std::vector<int32_t>& h, const DevBuf<int32_t>& d, size_t n) {
+        h.assign(n, 0);
+        return n ? cudaMemcpyAsync(h.data(), d.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c->stream) : cudaSuccess;
+    };
+    std::vector<int32_t> tri, dofOff, refV, vfOff, vf, rowOff, rowSrc, adjOff, adjRow, syOff, syV;
+    LF_TRY_CUDA(c, fetch(tri, c->d_tri, 3 * (size_t)T));
+    LF_TRY_CUDA(c, fetch(dofOff, c->d_dofOff, np + 1));
+    LF_TRY_CUDA(c, fetch(vfOff, c->d_vfOff, V + 1));
+    LF_TRY_CUDA(c, fetch(vf, c->d_vf, 3 * (size_t)T));
+    LF_TRY_CUDA(c, fetch(syOff, c->d_syncOff, c->nSync ? c->nSync + 1 : 0));
+    LF_TRY_CUDA(c, fetch(rowOff, c->d_interpOff, c->nInterpRows ? V + 1 : 0));
+    LF_TRY_CUDA(c, fetch(adjOff, c->d_adjOff, V + 1));
+    LF_TRY_CUDA(c, cudaStreamSynchronize(c->stream));
+    LF_TRY_CUDA(c, fetch(refV, c->d_refVertex, dofOff[np]));
+    LF_TRY_CUDA(c, fetch(syV, c->d_syncVertex, c->nSync ? syOff[c->nSync] : 0));
+    LF_TRY_CUDA(c, fetch(rowSrc, c->d_interpSrc, c->nInterpRows ? rowOff[V] : 0));
+    LF_TRY_CUDA(c, fetch(adjRow, c->d_adjRow, adjOff[V]));
+    LF_TRY_CUDA(c, cudaStreamSynchronize(c->stream));
+    c->sweepState = -1;
+    auto isRow = [&](int v) { return c->nInterpRows && rowOff[v + 1] > rowOff[v]; };
+    for (int32_t q : rowSrc)
+        if (isRow(q)) return LF_OK;
+    std::vector<int32_t> sync(V, -1);
+    for (int g = 0; g < c->nSync; ++g) {
+        if (syOff[g + 1] - syOff[g] < 2) continue;  // k_sync_shared leaves it alone
+        for (int k = syOff[g]; k < syOff[g + 1]; ++k) {
+            if (sync[syV[k]] >= 0) return LF_OK;
+            sync[syV[k]] = g;
+        }
+    }
+    constexpr size_t kMostTriangles = size_t(8) << 20;  // 128 MB of lists
+    constexpr size_t kSweepMostWhole = 64;
+    c->sweepMaxVerts = 1;
+    c->sweepWhole.clear();
+    std::vector<int32_t> listOf(np), avOff{0}, av, atOff{0}, slot(V, -1), seen(T, -1);
+    std::vector<int4> at;
+    for (int j = 0; j < np; ++j) {
+        const auto* r0 = refV.data();
+        const int b = dofOff[j], n = dofOff[j + 1] - b;
+        if (j > 0 && listOf[j - 1] >= 0 && n == b - dofOff[j - 1] && std::equal(r0 + b, r0 + b + n, r0 + dofOff[j - 1])) {
+            listOf[j] = listOf[j - 1];  // another axis of the same vertices
+            continue;
+        }
+        const int l = static_cast<int>(avOff.size()) - 1;
+        listOf[j] = l;
+        const size_t first = av.size();
+        auto add = [&](int v) {
+            if (slot[v] >= 0) return;
+            slot[v] = static_cast<int32_t>(av.size() - first);
+            av.push_back(v);
+        };
+        auto addWithGroup = [&](int v) {
+            if (sync[v] < 0) return add(v);
+            for (int k = syOff[sync[v]]; k < syOff[sync[v] + 1]; ++k) add(syV[k]);
+        };
+        for (int r = b; r < b + n; ++r) {
+            addWithGroup(refV[r]);
+            for (int k = adjOff[refV[r]]; k < adjOff[refV[r] + 1]; ++k) addWithGroup(adjRow[k]);
+        }
+        if (av.size() - first > (size_t)kSweepMaxVerts) {
+            for (size_t i = first; i < av.size(); ++i) slot[av[i]] = -1;
+            av.resize(first);
+            listOf[j] = -1;
+            c->sweepWhole.push_back(j);
+            if (c->sweepWhole.size() > kSweepMostWhole) return LF_OK;
+            continue;
+        }
+        for (size_t i = first; i < av.size(); ++i)
+            for (int k = vfOff[av[i]]; k < vfOff[av[i] + 1]; ++k) {
+                const int f = vf[k] / 3;
+                if (seen[f] == l) continue;
+                seen[f] = l;
+                auto code = [&](int q) { const int v = tri[3 * (size_t)f + q]; return slot[v] >= 0 ? slot[v] : ~v; };
+                at.push_back(make_int4(code(0), code(1), code(2), f));
+            }
+        for (size_t i = first; i < av.size(); ++i) slot[av[i]] = -1;
+        if (at.size() > kMostTriangles) return LF_OK;
+        c->sweepMaxVerts = std::max(c->sweepMaxVerts, static_cast<int>(av.size() - first));
+        avOff.push_back(static_cast<int32_t>(av.size()));
+        atOff.push_back(static_cast<int32_t>(at.size()));
+    }
+    if (at.empty()) at.push_back(make_int4(0, 0, 0, 0));
+    if (av.empty()) av.push_back(0);
+    LF_TRY_CUDA(c, upload(c->d_swList, listOf.data(), listOf.size(), c->stream));
+    LF_TRY_CUDA(c, upload(c->d_swAvOff, avOff.data(), avOff.size(), c->stream));
+    LF_TRY_CUDA(c, upload(c->d_swAv, av.data(), av.size(), c->stream));
+    LF_TRY_CUDA(c, upload(c->d_swAtOff, atOff.data(), atOff.size(), c->stream));
+    LF_TRY_CUDA(c, upload(c->d_swAt, at.data(), at.size(), c->stream));
+    LF_TRY_CUDA(c, upload(c->d_swSync, sync.data(), sync.size(), c->stream));
+    LF_TRY_CUDA(c, c->d_swSrc.reserve(3 * (size_t)V));
+    LF_TRY_CUDA(c, cudaStreamSynchronize(c->stream));
+    c->sweepState = 1;
+    return LF_OK;
+}
+
+// The whole finite-difference sweep at once (stateless scatter): base scatter
+// and crossing parities at the parameters, one launch over all passes, and the
+// positions of the last pass left behind.
+static lf_status sweep_side_by_side(lf_ctx* c) {
+    const double h = 1.0;  // constraint_handler.cpp:54
+    const int n = c->nCons;
+    LF_TRY_CUDA(c, c->d_swPre.reserve(n));
+    LF_RET_IF(scatter(c, c->d_cPar0.p, c->d_swSrc.p));
+    const int slices = std::max(1, std::min(cdiv(c->T, 2 * kCrossThreads), cdiv(148 * 8, n)));
+    k_classify_prep<<<cdiv(n, 128), 128, 0, c->stream>>>(n, c->d_cMid.p, c->G, c->bottomDepth, c->labelGrid,
+                                                         c->d_swPre.p, c->d_clsMask.p);
+    k_classify_cross<<<dim3(n, slices), kCrossThreads, 0, c->stream>>>(n, c->d_cMid.p, c->T, cdiv(c->T, slices),
+                                                                        c->d_faceGroup.p, c->d_tri.p, c->d_pos.p,
+                                                                        c->d_swPre.p, c->d_clsMask.p);
+    const SweepTables t{c->d_swList.p, c->d_swAvOff.p, c->d_swAv.p, c->d_swAtOff.p, c->d_swAt.p, c->d_swSrc.p,
+                        c->d_pos.p, c->d_dofOff.p, c->d_refVertex.p, c->d_refAxis.p, c->d_refScale.p,
+                        c->nInterpRows ? c->d_interpOff.p : nullptr, c->d_interpSrc.p, c->d_interpW.p, c->d_swSync.p,
+                        c->d_syncOff.p, c->d_syncVertex.p, c->d_tri.p, c->d_faceGroup.p};
+    const size_t smem = sizeof(double) * (3 * (size_t)c->sweepMaxVerts + 2 * (size_t)n);
+    LF_TRY_CUDA(c, cudaFuncSetAttribute(k_constraint_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)(sizeof(double) * (3 * kSweepMaxVerts + 2 * kSweepMaxPoints))));
+    k_constraint_sweep<<<dim3(c->np, 2), kSweepThreads, smem, c->stream>>>(
+        t, c->np, c->d_cPar0.p, h, n, c->d_cMid.p, c->d_swPre.p, c->d_clsMask.p, c->d_cGroup.p, c->d_cThick.p,
+        c->consWeight, c->sweepMaxVerts, c->d_cFp.p, c->d_cFm.p);
+    for (int j : c->sweepWhole)
+        for (int minus = 0; minus < 2; ++minus) {
+            k_constraint_step<<<1, 32, 0, c->stream>>>(c->d_cPar.p, c->d_cPar0.p, j, h, minus);
+            LF_RET_IF(constraint_eval_dev(c, (minus ? c->d_cFm.p : c->d_cFp.p) + j));
+            if (minus) k_constraint_step<<<1, 32, 0, c->stream>>>(c->d_cPar.p, c->d_cPar0.p, j, h, 2);
+            c->counters.launches += 1 + minus;
+        }
+    k_constraint_fd<<<cdiv(c->np, 256), 256, 0, c->stream>>>(c->np, c->d_cFp.p, c->d_cFm.p, h, c->consWeight,
+                                                              c->d_cGrad.p);
+    k_constraint_step<<<1, 32, 0, c->stream>>>(c->d_cPar.p, c->d_cPar0.p, c->np - 1, h, 1);
+    LF_RET_IF(scatter(c, c->d_cPar.p));
+    c->counters.launches += 5;
+    LF_CHECK_LAUNCH(c);
+    return LF_OK;
+}
+
 extern "C" lf_status lf_constraint_gradient(lf_ctx* c, const double* params, double* grad) {
     LF_RET_IF(model_ready(c));
     if (c->np > 0 && !grad) return fail(c, LF_EINVAL, "null grad");
@@ -2936,8 +3095,8 @@ extern "C" lf_status lf_constraint_gradient(lf_ctx* c, const double* params, dou
     LF_TRY_CUDA(c, c->d_cFm.reserve(c->np));
     LF_TRY_CUDA(c, c->d_cGrad.reserve(c->np));
     LF_TRY_CUDA(c, upload(c->d_grpTriOffDev, c->grpTriOff.data(), c->grpTriOff.size(), c->stream));
-    // The 2 np passes are sequential (each scatter starts from the positions
-    // the previous one left, as the reference's model does) and each is a
+    // The 2 np passes are sequential unless the scatter is stateless (each starts
+    // from the positions the previous one left, as the reference's model does) and each is a
     // handful of short launches, so the sweep is replayed as one CUDA graph
     // after its first direct run.
     auto sweep = [c]() -> lf_status {
@@ -2956,9 +3115,15 @@ extern "C" lf_status lf_constraint_gradient(lf_ctx* c, const double* params, dou
         LF_CHECK_LAUNCH(c);
         return LF_OK;
     };
+    // A stateless scatter makes the passes independent: all of them side by side
+    const bool independent =
+        c->statelessScatter && c->G <= 64 && c->nCons > 0 && c->nCons <= kSweepMaxPoints && c->T > 0;
+    if (independent) LF_RET_IF(sweep_tables(c));
     // graph replay up to 4096 parameters (about 66k graph nodes); beyond that
     // the capture itself would cost more than the launches it saves
-    if (c->np <= 4096)
+    if (independent && c->sweepState == 1)
+        LF_RET_IF(sweep_side_by_side(c));
+    else if (c->np <= 4096)
         LF_RET_IF(run_cached(c, c->gCons, c->d_cPar0.p, c->d_cFp.p, c->d_cGrad.p, sweep, true));
     else
         LF_RET_IF(sweep());
