@@ -1701,7 +1701,9 @@ static int gradient_set(lf_ctx* c, const StationSet& s, const double* gcoef, con
         fork = false;
     }
     int ev = prof_begin(c, c->evGrad, c->nGrad);
-    k_gradient_warp_fp64<<<dim3(fblocks, nch), 32 * kGradWarpsPerBlock, 0, c->stream>>>(
+    const auto fp64 = !mcoef ? k_gradient_warp_fp64<true, false>
+                             : (!gcoef ? k_gradient_warp_fp64<false, true> : k_gradient_warp_fp64<true, true>);
+    fp64<<<dim3(fblocks, nch), 32 * kGradWarpsPerBlock, 0, c->stream>>>(
         c->T, c->d_gc.p, s.n, s.d_xyz.p, gcoef, mcoef, s.d_tileBox.p, c->d_faceGroup.p, c->d_groups.p, c->fdir, tau,
         c->d_gradFacets.p, c->nGradFacets, tpc, grpSta, grpTile, c->d_partGrad.p + (size_t)slot0 * 9 * c->T);
     prof_end(c, c->evGrad, ev);
@@ -1838,7 +1840,7 @@ static lf_status gradient_all(lf_ctx* c, const double* d_params, double* d_grad)
             c->counters.launches++;
         }
         if (c->nInterpRows > 0) {
-            k_interp_adjoint<<<cdiv(c->V, 256), 256, 0, c->stream>>>(c->V, c->d_interpOff.p, c->d_adjOff.p,
+            k_interp_adjoint<<<cdiv(c->V, kAdjointThreads / 32), kAdjointThreads, 0, c->stream>>>(c->V, c->d_interpOff.p, c->d_adjOff.p,
                                                                      c->d_adjRow.p, c->d_adjW.p, c->d_vgrad.p,
                                                                      c->d_vgrad2.p);
             c->counters.launches++;
@@ -2631,38 +2633,42 @@ extern "C" lf_status lf_jacobian(lf_ctx* c, const double* params, int which, dou
                                                              c->d_groups.p, c->d_faceNeeds.p, which == LF_GRAVITY,
                                                              which == LF_MAGNETIC, c->fdir, c->d_gc.p);
     LF_CHECK_LAUNCH(c);
-    std::vector<double> ones(s.n, 1.0);
-    LF_TRY_CUDA(c, upload(c->d_ones, ones.data(), ones.size(), c->stream));
     int np = std::max(c->np, 1);
     // stations per batch so that the partial buffer stays below ~256 MB
     size_t per = (size_t)9 * c->T * sizeof(double);
     int batch = static_cast<int>(std::max<size_t>(1, std::min<size_t>({(size_t)s.n, ((size_t)256 << 20) / per, (size_t)65535})));
+    // Rows in caller order on the device, copied once straight into J, while
+    // they fit 256 MB; longer Jacobians go batch by batch through host rows.
+    const bool whole = (size_t)s.n * np * sizeof(double) <= ((size_t)256 << 20);
     LF_TRY_CUDA(c, c->d_partGrad.reserve((size_t)batch * 9 * c->T));
-    LF_TRY_CUDA(c, c->d_jac.reserve((size_t)batch * np));
+    LF_TRY_CUDA(c, c->d_jac.reserve((size_t)(whole ? s.n : batch) * np));
     std::vector<double> rows;
     for (int s0 = 0; s0 < s.n; s0 += batch) {
         int nb = std::min(batch, s.n - s0);
-        dim3 grid(cdiv(c->T, kGradThreads), nb);
-        const double* g1 = which == LF_GRAVITY ? c->d_ones.p : nullptr;
-        const double* m1 = which == LF_MAGNETIC ? c->d_ones.p : nullptr;
-        k_gradient_fp64<<<grid, kGradThreads, 0, c->stream>>>(
-            c->T, c->d_gc.p, nb, s.d_xyz.p + 3 * (size_t)s0, g1, m1, 1, c->d_faceGroup.p, c->d_groups.p, c->fdir,
-            c->d_partGrad.p);
+        const auto kernel = which == LF_GRAVITY ? k_gradient_fp64<true> : k_gradient_fp64<false>;
+        kernel<<<dim3(cdiv(c->T, kGradThreads), nb), kGradThreads, 0, c->stream>>>(
+            c->T, c->d_gc.p, s.d_xyz.p + 3 * (size_t)s0, c->d_faceGroup.p, c->d_groups.p, c->fdir, c->d_partGrad.p);
         if (c->np > 0) {
             dim3 g2(cdiv(c->np, 128), nb);
-            k_jacobian_gather<<<g2, 128, 0, c->stream>>>(nb, c->np, c->d_dofOff.p, c->d_refVertex.p, c->d_refAxis.p,
-                                                         c->d_refScale.p, c->d_vfOff.p, c->d_vf.p, c->T,
-                                                         c->d_partGrad.p, c->d_jac.p, c->np);
-            rows.resize((size_t)nb * c->np);
-            LF_TRY_CUDA(c, cudaMemcpyAsync(rows.data(), c->d_jac.p, sizeof(double) * (size_t)nb * c->np,
-                                           cudaMemcpyDeviceToHost, c->stream));
-            LF_TRY_CUDA(c, cudaStreamSynchronize(c->stream));
-            for (int r = 0; r < nb; ++r)
-                std::copy(rows.begin() + (size_t)r * c->np, rows.begin() + (size_t)(r + 1) * c->np,
-                          J + (size_t)s.perm[s0 + r] * c->np);
+            k_jacobian_gather<<<g2, 128, 0, c->stream>>>(nb, c->np, whole ? s.d_perm.p + s0 : nullptr, c->d_dofOff.p,
+                                                         c->d_refVertex.p, c->d_refAxis.p, c->d_refScale.p,
+                                                         c->d_vfOff.p, c->d_vf.p, c->T, c->d_partGrad.p, c->d_jac.p,
+                                                         c->np);
+            if (!whole) {
+                rows.resize((size_t)nb * c->np);
+                LF_TRY_CUDA(c, cudaMemcpyAsync(rows.data(), c->d_jac.p, sizeof(double) * (size_t)nb * c->np,
+                                               cudaMemcpyDeviceToHost, c->stream));
+                LF_TRY_CUDA(c, cudaStreamSynchronize(c->stream));
+                for (int r = 0; r < nb; ++r)
+                    std::copy(rows.begin() + (size_t)r * c->np, rows.begin() + (size_t)(r + 1) * c->np,
+                              J + (size_t)s.perm[s0 + r] * c->np);
+            }
         }
         LF_CHECK_LAUNCH(c);
     }
+    if (whole && c->np > 0)
+        LF_TRY_CUDA(c, cudaMemcpyAsync(J, c->d_jac.p, sizeof(double) * (size_t)s.n * c->np, cudaMemcpyDeviceToHost,
+                                       c->stream));
     LF_TRY_CUDA(c, cudaStreamSynchronize(c->stream));
     return LF_OK;
 }

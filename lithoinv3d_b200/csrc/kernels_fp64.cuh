@@ -914,10 +914,12 @@ __device__ __forceinline__ NearTerms gradient_near_terms(double x, double y, dou
 // (q = r1 - (r1.e) e = -d_perp n - z zhat and e x r1 = z n - d_perp zhat in
 // the facet's frame), so the terms of a vertex's two edges are added before
 // the division by its distance.  Away from the facet (every v = L / (d1 + d2)
-// below 1/2, see pair_forward_fp64) 1 / (d1 + d2) and W = 2 L / ((d1 + d2)^2 -
-// L^2) share one reciprocal and the polynomials replace the library's log1p
-// and atan2; other pairs take gradient_near_terms.  233 FP64 instructions per
-// pair (ncu) against more than 700 through the library functions.
+// below 1/2, see pair_forward_fp64) W = 2 L / ((d1 + d2)^2 - L^2) and the
+// polynomials replace the library's log1p and atan2; other pairs take
+// gradient_near_terms.  About 230 FP64 instructions per pair against more than
+// 700 through the library functions.  Gravity Jacobian of a 1,280-facet body
+// against extended precision: 3.5e-13 through the library functions, 3.4e-13
+// here (3.6e-13 without the corrected quotients).
 template <bool GZ, bool TMI>
 __device__ __forceinline__ void pair_gradient_fp64(const double* C, double gsn, double ms, double ox, double oy,
                                                    double oz, double gco, double mco, GradAcc& A) {
@@ -937,15 +939,20 @@ __device__ __forceinline__ void pair_gradient_fp64(const double* C, double gsn, 
     const double la = sqrt_inv64(a2, &ia), lb = sqrt_inv64(b2, &ib), lc = sqrt_inv64(c2, &ic);
     const double D0 = la + lb, D1 = lb + lc, D2 = lc + la;
     const double m0 = fma(D0, D0, -L0 * L0), m1 = fma(D1, D1, -L1 * L1), m2 = fma(D2, D2, -L2 * L2);
-    const double g0 = rcp_pos64(D0 * m0), g1 = rcp_pos64(D1 * m1), g2 = rcp_pos64(D2 * m2);
-    const double v0 = L0 * (g0 * m0), v1 = L1 * (g1 * m1), v2 = L2 * (g2 * m2);
+    const double q0 = rcp_pos64(D0), q1 = rcp_pos64(D1), q2 = rcp_pos64(D2);
+    double v0 = L0 * q0, v1 = L1 * q1, v2 = L2 * q2;
+    if (GZ && !TMI) {  // the gz terms cancel: quotients to half an ulp
+        v0 = fma(fma(-v0, D0, L0), q0, v0);
+        v1 = fma(fma(-v1, D1, L1), q1, v1);
+        v2 = fma(fma(-v2, D2, L2), q2, v2);
+    }
     const int vmax = max(__double2hiint(v0), max(__double2hiint(v1), __double2hiint(v2)));
     double om, l0, l1, l2, W0, W1, W2;
     bool lv0 = true, lv1 = true, lv2 = true;
     if (vmax < 0x3fe00000) {  // every v < 1/2
-        W0 = (L0 + L0) * (g0 * D0);
-        W1 = (L1 + L1) * (g1 * D1);
-        W2 = (L2 + L2) * (g2 * D2);
+        W0 = (L0 + L0) * rcp_pos64(m0);
+        W1 = (L1 + L1) * rcp_pos64(m1);
+        W2 = (L2 + L2) * rcp_pos64(m2);
         // ra . rb = (a2 + b2 - L^2) / 2
         const double dab = 0.5 * fma(-L0, L0, a2 + b2), dbc = 0.5 * fma(-L1, L1, b2 + c2),
                      dac = 0.5 * fma(-L2, L2, c2 + a2);
@@ -1023,35 +1030,29 @@ __device__ __forceinline__ bool facet_grad_active(const double* C) {
     return (flags & 1) && (flags & 2) && (C[GC_GS] != 0.0 || C[GC_MS] != 0.0);
 }
 
-// Per-station facet gradients for dense Jacobian rows.  Grid: x = facet
-// warps (one facet per thread), y = station chunks of stations_per_chunk
-// consecutive stations; part layout [chunk][9][T] (vertex a xyz, b xyz,
-// c xyz; global frame).  Stations are warp-uniform loads.
-__global__ void __launch_bounds__(32) k_gradient_fp64(int T, const double* __restrict__ gc, int S,
-                                                      const double* __restrict__ sta, const double* __restrict__ gcoef,
-                                                      const double* __restrict__ mcoef, int stations_per_chunk,
+// Per-station facet gradients for dense Jacobian rows of one data type (GZ:
+// gravity, else TMI; unit adjoints).  Grid: x = facet warps (one facet per
+// thread), y = stations; part layout [station][9][T] (vertex a xyz, b xyz, c
+// xyz; global frame).  Stations are warp-uniform loads.
+template <bool GZ>
+__global__ void __launch_bounds__(32) k_gradient_fp64(int T, const double* __restrict__ gc,
+                                                      const double* __restrict__ sta,
                                                       const int16_t* __restrict__ face_group,
                                                       const GroupConst* __restrict__ groups, d3 fdir,
                                                       double* __restrict__ part) {
-    int f = blockIdx.x * blockDim.x + threadIdx.x;
-    int chunk = blockIdx.y;
-    int sb = chunk * stations_per_chunk, se = min(S, sb + stations_per_chunk);
+    const int f = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
     if (f >= T) return;
     double C[NGC];
 #pragma unroll
     for (int k = 0; k < NGC; ++k) C[k] = gc[(size_t)k * T + f];
-    const bool active = facet_grad_active(C);
     double outv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (active) {
+    if (facet_grad_active(C)) {
         GradAcc A;
         grad_acc_zero(A);
-        const double gsn = C[GC_GS], ms = C[GC_MS];
-        for (int j = sb; j < se; ++j)
-            pair_gradient_fp64<true, true>(C, gsn, ms, sta[3 * j], sta[3 * j + 1], sta[3 * j + 2], gcoef ? gcoef[j] : 0.0,
-                               mcoef ? mcoef[j] : 0.0, A);
+        pair_gradient_fp64<GZ, !GZ>(C, C[GC_GS], C[GC_MS], sta[3 * j], sta[3 * j + 1], sta[3 * j + 2], 1.0, 1.0, A);
         grad_finalize(C, A, groups[face_group[f]], fdir, outv);
     }
-    for (int k = 0; k < 9; ++k) part[((size_t)chunk * 9 + k) * T + f] = outv[k];
+    for (int k = 0; k < 9; ++k) part[((size_t)j * 9 + k) * T + f] = outv[k];
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -1103,14 +1104,16 @@ __device__ __forceinline__ void grad_acc_warp_sum(GradAcc& A, double* row) {
 // the tile's stations in turn; per-lane sums are reduced across the warp
 // once per facet and lane 0 finalises.  The work of a facet is spread over
 // 32 lanes, so facets with many near tiles leave no long tail behind.
+// GZ / TMI: which adjoints there are (gcoef, mcoef not null).
 // Warps run over `facets` (those with a DOF vertex); grid.y splits the
 // station tiles into chunks of tiles_per_chunk so that a model with few such
 // facets still fills the GPU.  part layout [chunk][9][T].
 // FP64 pipe 65 % busy at 12 warps per SM (168 registers, of which 56 hold the
 // sums): 24.6 M pairs (8,308 facets, 2,964 stations) took 1,131 us with the
-// library functions, 489 us now; a 1,280-facet body under 1,600 stations 115
-// and 57 us.  Two CTAs per SM (no spill) 523 us, four (128 registers) 539;
+// library functions, 480 us now; a 1,280-facet body under 1,600 stations 115
+// and 55 us.  Two CTAs per SM (no spill) 523 us, four (128 registers) 539;
 // CTAs of one or two warps no different.
+template <bool GZ, bool TMI>
 __global__ void __launch_bounds__(128, 3) k_gradient_warp_fp64(int T, const double* __restrict__ gc, int S,
                                                             const double* __restrict__ sta,
                                                             const double* __restrict__ gcoef,
@@ -1163,8 +1166,8 @@ __global__ void __launch_bounds__(128, 3) k_gradient_warp_fp64(int T, const doub
                 for (int k = 0; k < kStationTile; k += 32) {
                     const int j = s0 + k + lane;
                     if (j < S)
-                        pair_gradient_fp64<true, true>(C, gsn, ms, sta[3 * j], sta[3 * j + 1], sta[3 * j + 2],
-                                           gcoef ? gcoef[j] : 0.0, mcoef ? mcoef[j] : 0.0, A);
+                        pair_gradient_fp64<GZ, TMI>(C, gsn, ms, sta[3 * j], sta[3 * j + 1], sta[3 * j + 2],
+                                                    GZ ? gcoef[j] : 0.0, TMI ? mcoef[j] : 0.0, A);
                 }
             }
         }
@@ -1305,25 +1308,50 @@ __global__ void k_dof_gather(int np, const int32_t* __restrict__ dof_off, const 
 // interpolation's transpose, out of place: a source receives w x the
 // gradient of each row it feeds, a row keeps nothing (its position was
 // overwritten), every other vertex keeps its own.  Fixed summation order,
-// no atomics.
-__global__ void k_interp_adjoint(int V, const int32_t* __restrict__ interp_off, const int32_t* __restrict__ adj_off,
-                                 const int32_t* __restrict__ adj_row, const double* __restrict__ adj_w,
-                                 const double* __restrict__ vg, double* __restrict__ out) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= V) return;
-    const bool row = interp_off[v + 1] > interp_off[v];
-    double g0 = row ? 0.0 : vg[3 * (size_t)v], g1 = row ? 0.0 : vg[3 * (size_t)v + 1],
-           g2 = row ? 0.0 : vg[3 * (size_t)v + 2];
-    for (int k = adj_off[v]; k < adj_off[v + 1]; ++k) {
-        const double w = adj_w[k];
-        const double* q = vg + 3 * (size_t)adj_row[k];
-        g0 += w * q[0];
-        g1 += w * q[1];
-        g2 += w * q[2];
+// no atomics.  A warp per vertex, lanes over its entries; a control point that
+// feeds more than kAdjointHeavy rows (a few drive thousands) takes the whole
+// CTA.  106,000 vertices, a few sources with tens of thousands of rows between them: 3.8 ms
+// with a thread per vertex, well under 0.1 ms now.
+constexpr int kAdjointHeavy = 512, kAdjointThreads = 256;
+__global__ void __launch_bounds__(kAdjointThreads) k_interp_adjoint(
+    int V, const int32_t* __restrict__ interp_off, const int32_t* __restrict__ adj_off,
+    const int32_t* __restrict__ adj_row, const double* __restrict__ adj_w, const double* __restrict__ vg,
+    double* __restrict__ out) {
+    constexpr int kWarps = kAdjointThreads / 32;
+    __shared__ double part[kWarps][3];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, first = blockIdx.x * kWarps;
+    auto sum = [&](int b, int e, int start, int step) {
+        d3 g = mk3(0.0, 0.0, 0.0);
+        for (int k = b + start; k < e; k += step) {
+            const double w = adj_w[k];
+            const double* q = vg + 3 * (size_t)adj_row[k];
+            g = mk3(g.x + w * q[0], g.y + w * q[1], g.z + w * q[2]);
+        }
+        return mk3(warp_sum(g.x), warp_sum(g.y), warp_sum(g.z));
+    };
+    auto store = [&](int v, d3 g) {
+        const bool row = interp_off[v + 1] > interp_off[v];
+        for (int k = 0; k < 3; ++k)
+            out[3 * (size_t)v + k] = (row ? 0.0 : vg[3 * (size_t)v + k]) + (k == 0 ? g.x : k == 1 ? g.y : g.z);
+    };
+    auto heavy = [&](int v) { return v < V && adj_off[v + 1] - adj_off[v] > kAdjointHeavy; };
+    const int mine = first + warp;
+    if (mine < V && !heavy(mine)) {  // warp-uniform
+        const d3 g = sum(adj_off[mine], adj_off[mine + 1], lane, 32);
+        if (lane == 0) store(mine, g);
     }
-    out[3 * (size_t)v] = g0;
-    out[3 * (size_t)v + 1] = g1;
-    out[3 * (size_t)v + 2] = g2;
+    for (int v = first; v < first + kWarps; ++v) {
+        if (!heavy(v)) continue;  // block-uniform
+        const d3 g = sum(adj_off[v], adj_off[v + 1], (int)threadIdx.x, kAdjointThreads);
+        if (lane == 0) { part[warp][0] = g.x; part[warp][1] = g.y; part[warp][2] = g.z; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            d3 t = mk3(0.0, 0.0, 0.0);
+            for (int w = 0; w < kWarps; ++w) t = t + mk3(part[w][0], part[w][1], part[w][2]);
+            store(v, t);
+        }
+        __syncthreads();
+    }
 }
 
 // y += a x over n doubles (the smoothness vertex gradient into the misfit's
@@ -1334,9 +1362,9 @@ __global__ void k_axpy(size_t n, double a, const double* __restrict__ x, double*
 }
 
 // Dense Jacobian rows from per-station facet partials (one chunk per
-// station): J[s][d] = sum_refs (sum_{(f,c) of v} part) * scale, with the
-// reference's |vertex gradient| < 1e-30 skip.
-__global__ void k_jacobian_gather(int nst, int np, const int32_t* __restrict__ dof_off,
+// station): J[row[s]][d] = sum_refs (sum_{(f,c) of v} part) * scale, with the
+// reference's |vertex gradient| < 1e-30 skip.  row nullptr: s itself.
+__global__ void k_jacobian_gather(int nst, int np, const int32_t* __restrict__ row, const int32_t* __restrict__ dof_off,
                                   const int32_t* __restrict__ ref_vertex, const uint8_t* __restrict__ ref_axis,
                                   const double* __restrict__ ref_scale, const int32_t* __restrict__ vf_off,
                                   const int32_t* __restrict__ vf, int T, const double* __restrict__ part,
@@ -1355,7 +1383,7 @@ __global__ void k_jacobian_gather(int nst, int np, const int32_t* __restrict__ d
         if (fabs(pg) < 1e-30) continue;
         acc += pg * ref_scale[r];
     }
-    J[(size_t)s * ld + d] = acc;
+    J[(size_t)(row ? row[s] : s) * ld + d] = acc;
 }
 
 // Final deterministic reduction of block partials and objective assembly:

@@ -8,7 +8,8 @@ s1 + d1 (stations at least 20 degrees off an edge's direction)."""
 import numpy as np
 import pytest
 
-from lithoinv3d_b200 import GRAVITY, MAGNETIC, synth
+from lithoinv3d_b200 import GATHER_CHAIN, GRAVITY, MAGNETIC, synth
+from lithoinv3d_b200.api import COLLAPSED_DROP
 from oracle_bindings import OracleModel
 
 pytestmark = pytest.mark.gpu
@@ -89,3 +90,48 @@ def test_derivative_routes(name, which):
     om.scatter(x)
     Jt = om.jacobian(sta, 2 + which)
     assert np.all(np.abs(J - Jt).max(1) <= 1e-6 * np.abs(Jt).max(1))
+
+
+def test_one_data_type_gradient():
+    """The gradient kernels for gravity or magnetic data alone against the sum
+    they split: the joint gradient is linear in the adjoints, and each station
+    set's part is computed by the kernel of its own (64 eps of the joint
+    gradient's largest entry per entry, several times the rounding of sums over
+    9 stations and 4 facets)."""
+    rng = np.random.default_rng(3)
+    sta = np.concatenate([CASES["quarter"], CASES["far"][1:]]) + rng.uniform(-1.0, 1.0, (14, 3))
+    p = synth.Problem("tetrahedron", [0.3], [0.02], [(V, F, synth.XYZ_FREE)], sta, sta)
+    model = p.build_model()
+    ctx = p.make_context(model)
+    x = model.assemble_parameters()
+    joint = ctx.objective_and_gradient(x)[1]
+    none = np.zeros((0, 3))
+    ctx.set_magnetic_data(none)
+    grav = ctx.objective_and_gradient(x)[1]
+    ctx.set_gravity_data(none)
+    ctx.set_magnetic_data(sta)
+    mag = ctx.objective_and_gradient(x)[1]
+    assert np.abs(grav + mag - joint).max() <= 64 * EPS * np.abs(joint).max()
+
+
+def test_heavy_interpolation_sources():
+    """Chain gather on a model whose control points drive thousands of rows (a
+    CTA per source; the other chain tests' feed few): the gradient along a random
+    step against a central difference of the objective (truncation and rounding
+    below 1e-5 of the sum of magnitudes at a step of 1e-3 m)."""
+    p = synth.voxel_contact_model(shape=(24, 24, 12), n_side=3, cp_stride=4)
+    model = p.build_model()
+    t = model.tables()
+    fed = np.bincount(t["interp_src"], minlength=len(t["pos"]))
+    assert fed.max() > 512
+    ctx = p.make_context(model)
+    ctx.set_gradient_gather(GATHER_CHAIN)
+    ctx.set_collapsed_facets(COLLAPSED_DROP)
+    ctx.set_scatter_stateless(True)
+    rng = np.random.default_rng(1)
+    x = model.assemble_parameters() + rng.normal(0.0, 3.0, model.n_dofs)
+    g = ctx.objective_and_gradient(x)[1]
+    step = rng.normal(0.0, 1.0, model.n_dofs)
+    h = 1e-3
+    fd = (ctx.objective(x + h * step) - ctx.objective(x - h * step)) / (2 * h)
+    assert abs(fd - g @ step) <= 1e-5 * np.abs(g * step).sum()
