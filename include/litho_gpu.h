@@ -289,6 +289,13 @@ lf_status lf_mlp_create(int device, int n_in, int width, int depth, int n_out, i
 void lf_mlp_destroy(lf_mlp* m);
 const char* lf_mlp_last_error(lf_mlp* m);
 lf_status lf_mlp_train_step(lf_mlp* m, const float* d_x, const float* d_y, float lr, float* loss);
+/* n_batches training steps on row batches of d_x [n_rows][n_in] and d_y
+ * [n_rows][n_out] (device, ready on every stream): batch b takes the rows
+ * rows[b * batch .. (b + 1) * batch) (host).  Same results as gathering the
+ * rows and calling lf_mlp_train_step; losses[b] (host) receives batch b's
+ * loss.  LF_EINVAL, with nothing trained, if a row number is out of range. */
+lf_status lf_mlp_train_rows(lf_mlp* m, const float* d_x, const float* d_y, long long n_rows, const long long* rows,
+                            int n_batches, float lr, float* losses);
 lf_status lf_mlp_predict(lf_mlp* m, const float* d_x, int rows, float* d_y);
 lf_status lf_mlp_param_count(lf_mlp* m, size_t* n);
 lf_status lf_mlp_get_params(lf_mlp* m, float* host);
@@ -303,8 +310,9 @@ lf_status lf_mlp_gradients(lf_mlp* m, const float* d_x, const float* d_y, float*
  *  LF_GEMM_TCGEN05_TMA: the same MMA fed by TMA (2-D tensor maps, 128-byte
  *    swizzle, no multicast) in a warp-specialised pipeline (one producer
  *    warp, one MMA warp, every warp in the epilogue);
- *  LF_GEMM_AUTO (default): per GEMM, LF_GEMM_TCGEN05_TMA for K >= 2048 and
- *    LF_GEMM_MMA_SYNC below (measured faster on each side of that line).
+ *  LF_GEMM_AUTO (default): per GEMM, LF_GEMM_TCGEN05_TMA for a deep K on
+ *    enough output tiles and LF_GEMM_MMA_SYNC otherwise (measured faster on
+ *    each side of that line).
  * All give the same results to FP32 summation order. */
 enum { LF_GEMM_TCGEN05 = 0, LF_GEMM_MMA_SYNC = 1, LF_GEMM_TCGEN05_TMA = 2, LF_GEMM_AUTO = 3 };
 lf_status lf_mlp_set_engine(lf_mlp* m, int engine);

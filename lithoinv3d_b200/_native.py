@@ -93,6 +93,8 @@ SIGNATURES = {
     "lf_mlp_destroy": (None, [_vp]),
     "lf_mlp_last_error": (C.c_char_p, [_vp]),
     "lf_mlp_train_step": (C.c_int, [_vp, C.c_void_p, C.c_void_p, C.c_float, C.POINTER(C.c_float)]),
+    "lf_mlp_train_rows": (C.c_int, [_vp, C.c_void_p, C.c_void_p, C.c_longlong, C.c_void_p, C.c_int, C.c_float,
+                                    C.c_void_p]),
     "lf_mlp_predict": (C.c_int, [_vp, C.c_void_p, C.c_int, C.c_void_p]),
     "lf_mlp_param_count": (C.c_int, [_vp, C.POINTER(C.c_size_t)]),
     "lf_mlp_get_params": (C.c_int, [_vp, C.c_void_p]),

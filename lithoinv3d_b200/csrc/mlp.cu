@@ -55,11 +55,14 @@ struct Buf {
     }
 };
 
+constexpr int kQueued = 32;  // training batches launched before the host waits
+
 struct Layer {
     int in = 0, out = 0;  // padded dims
     Buf<float> w, b, gw, gb, mw, vw, mb, vb;
     Buf<__nv_bfloat16> wb;  // bf16 copy [out][in]
     Buf<__nv_bfloat16> act;  // bf16 output activation [batch][out] (hidden layers)
+    Buf<__nv_bfloat16> dz;   // bf16 gradient of the output before the ReLU [batch][out]
 };
 
 }  // namespace
@@ -69,8 +72,12 @@ struct lf_mlp {
     cudaStream_t stream = nullptr;
     int n_in = 0, n_in_pad = 0, width = 0, depth = 0, n_out = 0, n_out_pad = 0, batch = 0;
     std::vector<Layer> layers;  // depth hidden + 1 output
-    Buf<__nv_bfloat16> xb, dz, dh;  // input, gradient buffers (bf16)
+    Buf<__nv_bfloat16> xb;  // input (bf16)
     Buf<float> pred, loss_blocks;
+    int n_loss = 0;           // loss blocks of one batch; loss_blocks holds kQueued batches
+    float* h_loss = nullptr;  // pinned: the loss blocks, then the GEMM error flag
+    Buf<long long> rows;      // row numbers of the queued batches, and their pinned host copy
+    long long* h_rows = nullptr;
     int step = 0;
     int engine = LF_GEMM_AUTO;  // lf_mlp_set_engine: per GEMM, TMA-fed tcgen05 for deep K, mma.sync otherwise
     std::string err;
@@ -162,18 +169,65 @@ static cudaError_t gemm_tma(cudaStream_t stream, int M, int N, int K, const __nv
     return cudaPeekAtLastError();
 }
 
-// LF_GEMM_AUTO: the TMA-fed tcgen05 kernel for deep reductions, where its
-// pipeline pays (measured on B200: 24.7 against 12.2 TFLOP/s at K = 8192 on
-// the network's 256 x 512 first layer, 757 against 290 at 4096^3), the
-// mma.sync kernel for the shallow ones (81 against 52 TFLOP/s at K = 256,
-// 14.0 against 8.9 at K = 512).
-constexpr int kAutoTmaMinK = 2048;
-static int auto_engine(int K) { return K >= kAutoTmaMinK && K % kTcBK == 0 ? LF_GEMM_TCGEN05_TMA : LF_GEMM_MMA_SYNC; }
+// LF_GEMM_AUTO: the TMA-fed tcgen05 kernel where a deep reduction has enough
+// 128 x 128 output tiles to fill a third of the SMs, the mma.sync kernel
+// otherwise: its 32 x 32 tiles spread a small product over the whole chip,
+// where one tcgen05 tile is a serial chain of K / 16 instructions on one SM.
+// Measured on B200, microseconds of a blocking call (20 of them its own),
+// mma.sync against tcgen05: 256 x 512 x 8192 39 / 90, 512 x 1024 x 8192
+// 79 / 91, 768 x 1024 x 8192 111 / 91, 2048 x 2048 x 8192 295 / 97; at K = 2048
+// 256 x 512 22 / 54, 1024 x 1024 41 / 54, 2048 x 2048 88 / 56.  Below K = 2048
+// tcgen05 stays behind (14.0 against 8.9 TFLOP/s at K = 512).
+constexpr int kAutoTmaMinK = 2048, kAutoTmaMinTiles = 48;
+static int auto_engine(int M, int N, int K) {
+    const bool tma = K >= kAutoTmaMinK && K % kTcBK == 0 && (long long)(M / kBM) * (N / kBN) >= kAutoTmaMinTiles;
+    return tma ? LF_GEMM_TCGEN05_TMA : LF_GEMM_MMA_SYNC;
+}
+
+// The mma.sync kernel's CTA tile: the largest that still gives every SM a
+// tile, 32 for what is smaller than that (a 256 x 512 layer is 8 tiles of 128
+// on 148 SMs, 128 tiles of 32).  Kernel times on B200: 256 x 512 x 512 9.5 ->
+// 3.8 us (tiles of 128, of 32), 256 x 512 x 1408 26 -> 6.9 us, 256 x 512 x 8192
+// 27 us (87 us in 128 x 256 tiles of the tcgen05 kernel); 1024 x 1024 x 1024
+// 36 -> 26 us a blocking call with tiles of 64.
+constexpr int kSms = 148;
+static int mma_tile(int M, int N, int K) {
+    if ((long long)(M / 128) * (N / 128) >= kSms) return 128;
+    return (long long)(M / 64) * (N / 64) >= kSms || K % MmaShape<32>::kBK ? 64 : 32;
+}
+
+template <int BT, bool A_T, bool B_T, int EPI>
+static cudaError_t launch_mma(cudaStream_t stream, int M, int N, int K, const __nv_bfloat16* A, int lda,
+                              const __nv_bfloat16* B, int ldb, const float* bias, float* Cf, __nv_bfloat16* Cb,
+                              int ldc, const __nv_bfloat16* y) {
+    using Sh = MmaShape<BT>;
+    static bool attr = false;  // per instantiation, per process
+    if (Sh::kSmem > 48 * 1024 && !attr) {
+        cudaError_t e = cudaFuncSetAttribute(k_gemm_bf16<BT, A_T, B_T, EPI>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem);
+        if (e != cudaSuccess) return e;
+        attr = true;
+    }
+    k_gemm_bf16<BT, A_T, B_T, EPI><<<dim3(N / BT, M / BT), Sh::kThreads, Sh::kSmem, stream>>>(K, A, lda, B, ldb, bias,
+                                                                                            Cf, Cb, ldc, y);
+    return cudaPeekAtLastError();  // left for the caller's launch check
+}
+
+template <bool A_T, bool B_T, int EPI>
+static cudaError_t gemm_mma(cudaStream_t stream, int M, int N, int K, const __nv_bfloat16* A, int lda,
+                            const __nv_bfloat16* B, int ldb, const float* bias, float* Cf, __nv_bfloat16* Cb, int ldc,
+                            const __nv_bfloat16* y = nullptr) {
+    switch (mma_tile(M, N, K)) {
+    case 128: return launch_mma<128, A_T, B_T, EPI>(stream, M, N, K, A, lda, B, ldb, bias, Cf, Cb, ldc, y);
+    case 64: return launch_mma<64, A_T, B_T, EPI>(stream, M, N, K, A, lda, B, ldb, bias, Cf, Cb, ldc, y);
+    default: return launch_mma<32, A_T, B_T, EPI>(stream, M, N, K, A, lda, B, ldb, bias, Cf, Cb, ldc, y);
+    }
+}
 
 template <bool A_T, bool B_T, int EPI>
 static cudaError_t gemm_on(int engine, cudaStream_t stream, int M, int N, int K, const __nv_bfloat16* A, int lda,
                            const __nv_bfloat16* B, int ldb, const float* bias, float* Cf, __nv_bfloat16* Cb, int ldc) {
-    if (engine == LF_GEMM_AUTO) engine = auto_engine(K);
+    if (engine == LF_GEMM_AUTO) engine = auto_engine(M, N, K);
     if (engine == LF_GEMM_TCGEN05_TMA) {
         if (N % 256 == 0)
             return gemm_tma<A_T, B_T, EPI, 256>(stream, M, N, K, A, lda, B, ldb, bias, Cf, Cb, ldc);
@@ -184,9 +238,7 @@ static cudaError_t gemm_on(int engine, cudaStream_t stream, int M, int N, int K,
             return gemm_tc<A_T, B_T, EPI, 256>(stream, M, N, K, A, lda, B, ldb, bias, Cf, Cb, ldc);
         return gemm_tc<A_T, B_T, EPI, 128>(stream, M, N, K, A, lda, B, ldb, bias, Cf, Cb, ldc);
     }
-    dim3 grid(N / kBN, M / kBM);
-    k_gemm_bf16<A_T, B_T, EPI><<<grid, kGemmThreads, 0, stream>>>(M, N, K, A, lda, B, ldb, bias, Cf, Cb, ldc);
-    return cudaPeekAtLastError();  // left for the caller's launch check
+    return gemm_mma<A_T, B_T, EPI>(stream, M, N, K, A, lda, B, ldb, bias, Cf, Cb, ldc);
 }
 
 template <bool A_T, bool B_T, int EPI>
@@ -196,12 +248,25 @@ static void gemm(lf_mlp* m, int M, int N, int K, const __nv_bfloat16* A, int lda
     if (e != cudaSuccess && m->err.empty()) m->err = std::string("gemm launch: ") + cudaGetErrorString(e);
 }
 
-// Reads and clears the tensor-core GEMM error flag (an mbarrier wait that
-// expired); synchronises the stream.
-static lf_status tc_check(lf_mlp* m) {
+// Waits for the stream; then the losses of the last n batches into losses[n],
+// and the tensor-core GEMM error flag (an mbarrier wait that expired), read
+// and cleared, where `tc`.
+static lf_status finish(lf_mlp* m, int n, float* losses, bool tc) {
     unsigned int flag = 0;
-    MLP_TRY(m, cudaMemcpyFromSymbolAsync(&flag, g_tc_gemm_error, sizeof(flag), 0, cudaMemcpyDeviceToHost, m->stream));
+    float* h_flag = m->h_loss + (size_t)kQueued * m->n_loss;
+    if (losses)
+        MLP_TRY(m, cudaMemcpyAsync(m->h_loss, m->loss_blocks.p, sizeof(float) * n * m->n_loss, cudaMemcpyDeviceToHost,
+                                   m->stream));
+    if (tc)
+        MLP_TRY(m, cudaMemcpyFromSymbolAsync(h_flag, g_tc_gemm_error, sizeof(flag), 0, cudaMemcpyDeviceToHost,
+                                             m->stream));
     MLP_TRY(m, cudaStreamSynchronize(m->stream));
+    for (int b = 0; losses && b < n; ++b) {
+        double s = 0.0;
+        for (int i = 0; i < m->n_loss; ++i) s += m->h_loss[(size_t)b * m->n_loss + i];
+        losses[b] = static_cast<float>(s);
+    }
+    if (tc) std::memcpy(&flag, h_flag, sizeof(flag));
     if (flag) {
         const unsigned int zero = 0;
         MLP_TRY(m, cudaMemcpyToSymbol(g_tc_gemm_error, &zero, sizeof(zero)));
@@ -260,21 +325,23 @@ extern "C" lf_status lf_mlp_create(int device, int n_in, int width, int depth, i
             if (e == cudaSuccess) e = b->alloc(L.out);
         if (e == cudaSuccess) e = L.wb.alloc(nw);
         if (e == cudaSuccess && l < depth) e = L.act.alloc((size_t)batch * L.out);
+        if (e == cudaSuccess) e = L.dz.alloc((size_t)batch * L.out);
         if (e == cudaSuccess) e = cudaMemcpy(L.w.p, w.data(), nw * sizeof(float), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(L.wb.p, wb.data(), nw * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) st = LF_ECUDA;
     }
     if (st == LF_OK) {
-        const int widest = std::max(std::max(m->n_in_pad, m->width), m->n_out_pad);
+        m->n_loss = cdiv_i((long long)batch * m->n_out_pad, 256);
         if (m->xb.alloc((size_t)batch * m->n_in_pad) != cudaSuccess ||
-            m->dz.alloc((size_t)batch * widest) != cudaSuccess || m->dh.alloc((size_t)batch * widest) != cudaSuccess ||
             m->pred.alloc((size_t)batch * m->n_out_pad) != cudaSuccess ||
-            m->loss_blocks.alloc(cdiv_i((long long)batch * m->n_out_pad, 256)) != cudaSuccess)
+            m->loss_blocks.alloc((size_t)kQueued * m->n_loss) != cudaSuccess ||
+            m->rows.alloc((size_t)kQueued * batch) != cudaSuccess ||
+            cudaMallocHost(&m->h_loss, sizeof(float) * ((size_t)kQueued * m->n_loss + 1)) != cudaSuccess ||
+            cudaMallocHost(&m->h_rows, sizeof(long long) * (size_t)kQueued * batch) != cudaSuccess)
             st = LF_ECUDA;
     }
     if (st != LF_OK) {
-        cudaStreamDestroy(m->stream);
-        delete m;
+        lf_mlp_destroy(m);
         return st;
     }
     *out = m;
@@ -286,22 +353,19 @@ extern "C" void lf_mlp_destroy(lf_mlp* m) {
     cudaSetDevice(m->device);
     cudaStreamSynchronize(m->stream);
     cudaStreamDestroy(m->stream);
+    if (m->h_loss) cudaFreeHost(m->h_loss);
+    if (m->h_rows) cudaFreeHost(m->h_rows);
     delete m;
 }
 
 extern "C" const char* lf_mlp_last_error(lf_mlp* m) { return m ? m->err.c_str() : "null network"; }
 
-// Input rows [rows][n_in] fp32 (device) -> padded bf16 [batch][n_in_pad].
-static lf_status load_input(lf_mlp* m, const float* d_x, int rows) {
-    MLP_TRY(m, cudaMemsetAsync(m->xb.p, 0, sizeof(__nv_bfloat16) * m->xb.n, m->stream));
-    if (m->n_in == m->n_in_pad) {
-        const size_t n = (size_t)rows * m->n_in;
-        k_to_bf16<<<cdiv_i(n, 256), 256, 0, m->stream>>>(n, d_x, m->xb.p);
-    } else {
-        for (int r = 0; r < rows; ++r)
-            k_to_bf16<<<cdiv_i(m->n_in, 256), 256, 0, m->stream>>>(m->n_in, d_x + (size_t)r * m->n_in,
-                                                                    m->xb.p + (size_t)r * m->n_in_pad);
-    }
+// The batch's input, n rows of d_x [][n_in] fp32 (device), the given ones or
+// the first -> padded bf16 [batch][n_in_pad].
+static lf_status load_input(lf_mlp* m, const float* d_x, int n, const long long* d_rows = nullptr) {
+    const bool vec = m->n_in % 4 == 0 && reinterpret_cast<uintptr_t>(d_x) % 16 == 0;
+    k_load_input<<<cdiv_i((long long)m->batch * m->n_in_pad, 4 * 256), 256, 0, m->stream>>>(
+        n, m->batch, m->n_in, m->n_in_pad, vec, d_x, d_rows, m->xb.p);
     return mlp_check_launch(m);
 }
 
@@ -321,61 +385,106 @@ static lf_status forward(lf_mlp* m) {
     return mlp_check_launch(m);
 }
 
-// Loss and parameter gradients for one batch (targets [batch][n_out] fp32).
-static lf_status backward(lf_mlp* m, const float* d_y, float* loss) {
-    const size_t np = (size_t)m->batch * m->n_out_pad;
-    const int nb = cdiv_i(np, 256);
-    k_mse<<<nb, 256, 0, m->stream>>>(m->batch, m->n_out_pad, m->n_out, m->pred.p, d_y, m->n_out, m->dz.p,
-                                     m->loss_blocks.p);
-    for (int l = m->depth; l >= 0; --l) {
-        Layer& L = m->layers[l];
-        const __nv_bfloat16* xin = l == 0 ? m->xb.p : m->layers[l - 1].act.p;
-        // dW [out][in] = dZ^T X: A = dZ stored [batch][out] = [K][M]; B = X [batch][in] = [K][N]
-        gemm<true, false, EPI_F32>(m, L.out, L.in, m->batch, m->dz.p, L.out, xin, L.in, nullptr, L.gw.p, nullptr, L.in);
-        k_colsum<<<cdiv_i(L.out, 128), 128, 0, m->stream>>>(m->batch, L.out, m->dz.p, L.gb.p);
-        if (l > 0) {
-            // dH [batch][in] = dZ W: A = dZ [batch][out], B = W [out][in] = [K][N]
-            gemm<false, false, EPI_BF16>(m, m->batch, L.in, L.out, m->dz.p, L.out, L.wb.p, L.in, nullptr, nullptr,
-                                         m->dh.p, L.in);
+static bool on_mma(const lf_mlp* m, int M, int N, int K) {
+    return m->engine == LF_GEMM_MMA_SYNC || (m->engine == LF_GEMM_AUTO && auto_engine(M, N, K) == LF_GEMM_MMA_SYNC);
+}
+
+// Loss (blocks of queue slot `slot`) and parameter gradients for one batch
+// (targets: rows of d_y [][n_out] fp32, the given ones or the first); with
+// `update` the gradients go straight into the Adam step.
+static lf_status backward(lf_mlp* m, const float* d_y, const Adam* update, const long long* d_rows = nullptr,
+                          int slot = 0) {
+    k_mse<<<m->n_loss, 256, 0, m->stream>>>(m->batch, m->n_out_pad, m->n_out, m->pred.p, d_y, d_rows,
+                                            m->n_out, m->layers[m->depth].dz.p,
+                                            m->loss_blocks.p + (size_t)slot * m->n_loss);
+    for (int l = m->depth; l > 0; --l) {
+        // dZ below: dH [batch][in] = dZ W (A = dZ [batch][out], B = W [out][in] = [K][N]), through the ReLU
+        Layer &L = m->layers[l], &P = m->layers[l - 1];
+        if (on_mma(m, m->batch, L.in, L.out)) {
+            gemm_mma<false, false, EPI_BF16_RELU_BWD>(m->stream, m->batch, L.in, L.out, L.dz.p, L.out, L.wb.p, L.in,
+                                                      nullptr, nullptr, P.dz.p, L.in, P.act.p);
+        } else {
+            gemm<false, false, EPI_BF16>(m, m->batch, L.in, L.out, L.dz.p, L.out, L.wb.p, L.in, nullptr, nullptr,
+                                         P.dz.p, L.in);
             const size_t n = (size_t)m->batch * L.in;
-            k_relu_bwd<<<cdiv_i(n, 256), 256, 0, m->stream>>>(n, xin, m->dh.p);
-            std::swap(m->dz.p, m->dh.p);
-            std::swap(m->dz.n, m->dh.n);
+            k_relu_bwd<<<cdiv_i(n, 256), 256, 0, m->stream>>>(n, P.act.p, P.dz.p);
         }
     }
-    lf_status st = mlp_check_launch(m);
-    if (st != LF_OK) return st;
-    if (loss) {
-        std::vector<float> lb(nb);
-        MLP_TRY(m, cudaMemcpyAsync(lb.data(), m->loss_blocks.p, sizeof(float) * nb, cudaMemcpyDeviceToHost, m->stream));
-        MLP_TRY(m, cudaStreamSynchronize(m->stream));
-        double s = 0.0;
-        for (float v : lb) s += v;
-        *loss = static_cast<float>(s);
+    bool grouped = true;
+    for (const Layer& L : m->layers) grouped = grouped && on_mma(m, L.out, L.in, m->batch);
+    if (grouped) {
+        for (int l0 = 0; l0 <= m->depth; l0 += kGradLayers) {
+            LayerGrads G{};
+            G.n = std::min(kGradLayers, m->depth + 1 - l0);
+            int blocks = 0;
+            for (int l = 0; l < G.n; ++l) {
+                Layer& L = m->layers[l0 + l];
+                G.layer[l] = {L.dz.p, l0 + l == 0 ? m->xb.p : m->layers[l0 + l - 1].act.p, L.w.p, L.gw.p, L.mw.p,
+                              L.vw.p, L.b.p, L.gb.p, L.mb.p, L.vb.p, L.wb.p, L.in, L.out, blocks};
+                blocks += (L.in / 64) * (L.out / 64) + L.out / 32;
+            }
+            if (update)
+                k_layer_grads<true><<<blocks, MmaShape<64>::kThreads, 0, m->stream>>>(G, m->batch, *update);
+            else
+                k_layer_grads<false><<<blocks, MmaShape<64>::kThreads, 0, m->stream>>>(G, m->batch, Adam{});
+        }
+    } else {
+        for (int l = m->depth; l >= 0; --l) {
+            Layer& L = m->layers[l];
+            const __nv_bfloat16* xin = l == 0 ? m->xb.p : m->layers[l - 1].act.p;
+            // dW [out][in] = dZ^T X: A = dZ stored [batch][out] = [K][M]; B = X [batch][in] = [K][N]
+            gemm<true, false, EPI_F32>(m, L.out, L.in, m->batch, L.dz.p, L.out, xin, L.in, nullptr, L.gw.p, nullptr,
+                                       L.in);
+            k_colsum<<<L.out / 32, 128, 0, m->stream>>>(m->batch, L.out, L.dz.p, L.gb.p);
+            if (!update) continue;
+            const size_t nw = (size_t)L.in * L.out;
+            k_adam<<<cdiv_i(nw, 256), 256, 0, m->stream>>>(nw, L.w.p, L.gw.p, L.mw.p, L.vw.p, *update, L.wb.p);
+            k_adam<<<cdiv_i(L.out, 256), 256, 0, m->stream>>>(L.out, L.b.p, L.gb.p, L.mb.p, L.vb.p, *update, nullptr);
+        }
     }
-    return LF_OK;
+    return mlp_check_launch(m);
+}
+
+// Queues one training step.
+static lf_status queue_step(lf_mlp* m, const float* d_x, const float* d_y, const long long* d_rows, int slot,
+                            float lr) {
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    const float t = (float)(m->step + 1);
+    const Adam adam{lr, b1, b2, eps, 1.f - std::pow(b1, t), 1.f - std::pow(b2, t)};
+    lf_status st = load_input(m, d_x, m->batch, d_rows);
+    if (st == LF_OK) st = forward(m);
+    if (st == LF_OK) st = backward(m, d_y, &adam, d_rows, slot);
+    if (st == LF_OK) ++m->step;
+    return st;
 }
 
 extern "C" lf_status lf_mlp_train_step(lf_mlp* m, const float* d_x, const float* d_y, float lr, float* loss) {
     if (!m || !d_x || !d_y || !(lr > 0.f)) return LF_EINVAL;
     cudaSetDevice(m->device);
-    lf_status st = load_input(m, d_x, m->batch);
-    if (st == LF_OK) st = forward(m);
-    if (st == LF_OK) st = backward(m, d_y, loss);
-    if (st != LF_OK) return st;
-    ++m->step;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-    for (Layer& L : m->layers) {
-        const size_t nw = (size_t)L.in * L.out;
-        k_adam<<<cdiv_i(nw, 256), 256, 0, m->stream>>>(nw, L.w.p, L.gw.p, L.mw.p, L.vw.p, lr, b1, b2, eps, c1, c2,
-                                                        L.wb.p);
-        k_adam<<<cdiv_i(L.out, 256), 256, 0, m->stream>>>(L.out, L.b.p, L.gb.p, L.mb.p, L.vb.p, lr, b1, b2, eps, c1, c2,
-                                                           nullptr);
+    const lf_status st = queue_step(m, d_x, d_y, nullptr, 0, lr);
+    const bool tc = m->engine != LF_GEMM_MMA_SYNC;
+    return st == LF_OK && (loss || tc) ? finish(m, 1, loss, tc) : st;
+}
+
+extern "C" lf_status lf_mlp_train_rows(lf_mlp* m, const float* d_x, const float* d_y, long long n_rows,
+                                       const long long* rows, int n_batches, float lr, float* losses) {
+    if (!m || !d_x || !d_y || n_rows < 0 || n_batches < 0 || (n_batches > 0 && (!rows || !losses)) || !(lr > 0.f))
+        return LF_EINVAL;
+    for (long long i = 0; i < (long long)n_batches * m->batch; ++i)
+        if (rows[i] < 0 || rows[i] >= n_rows) return LF_EINVAL;
+    cudaSetDevice(m->device);
+    for (int b0 = 0; b0 < n_batches; b0 += kQueued) {
+        const int nb = std::min(kQueued, n_batches - b0);
+        const size_t n = (size_t)nb * m->batch;
+        std::memcpy(m->h_rows, rows + (size_t)b0 * m->batch, sizeof(long long) * n);
+        MLP_TRY(m, cudaMemcpyAsync(m->rows.p, m->h_rows, sizeof(long long) * n, cudaMemcpyHostToDevice, m->stream));
+        lf_status st = LF_OK;
+        for (int b = 0; b < nb && st == LF_OK; ++b)
+            st = queue_step(m, d_x, d_y, m->rows.p + (size_t)b * m->batch, b, lr);
+        const lf_status done = finish(m, nb, losses + b0, m->engine != LF_GEMM_MMA_SYNC);  // always: h_rows is reused
+        if (st != LF_OK || done != LF_OK) return st != LF_OK ? st : done;
     }
-    st = mlp_check_launch(m);
-    if (st == LF_OK && m->engine != LF_GEMM_MMA_SYNC) st = tc_check(m);
-    return st;
+    return LF_OK;
 }
 
 extern "C" lf_status lf_mlp_predict(lf_mlp* m, const float* d_x, int rows, float* d_y) {
@@ -390,8 +499,7 @@ extern "C" lf_status lf_mlp_predict(lf_mlp* m, const float* d_x, int rows, float
                                      sizeof(float) * m->n_out_pad, sizeof(float) * m->n_out, nr,
                                      cudaMemcpyDeviceToDevice, m->stream));
     }
-    MLP_TRY(m, cudaStreamSynchronize(m->stream));
-    return m->engine != LF_GEMM_MMA_SYNC ? tc_check(m) : LF_OK;
+    return finish(m, 0, nullptr, m->engine != LF_GEMM_MMA_SYNC);
 }
 
 // Parameters in the unpadded order: for each layer W [out][in] then b [out].
@@ -410,7 +518,7 @@ extern "C" lf_status lf_mlp_param_count(lf_mlp* m, size_t* n) {
     return LF_OK;
 }
 
-// which: 0 weights, 1 gradients of the last lf_mlp_gradients / train step.
+// which: 0 weights, 1 gradients of the last lf_mlp_gradients.
 static lf_status copy_params(lf_mlp* m, int which, float* host) {
     size_t k = 0;
     for (int l = 0; l <= m->depth; ++l) {
@@ -467,8 +575,8 @@ extern "C" lf_status lf_mlp_gradients(lf_mlp* m, const float* d_x, const float* 
     cudaSetDevice(m->device);
     lf_status st = load_input(m, d_x, m->batch);
     if (st == LF_OK) st = forward(m);
-    if (st == LF_OK) st = backward(m, d_y, loss);
-    if (st == LF_OK && m->engine != LF_GEMM_MMA_SYNC) st = tc_check(m);
+    if (st == LF_OK) st = backward(m, d_y, nullptr);
+    if (st == LF_OK) st = finish(m, 1, loss, m->engine != LF_GEMM_MMA_SYNC);
     if (st == LF_OK && host_grads) st = copy_params(m, 1, host_grads);
     return st;
 }
@@ -489,7 +597,7 @@ extern "C" lf_status lf_mlp_set_engine(lf_mlp* m, int engine) {
 extern "C" lf_status lf_gemm_bf16(int engine, int a_trans, int b_trans, int epilogue, int M, int N, int K,
                                   const void* A, int lda, const void* B, int ldb, const float* bias, void* C, int ldc,
                                   void* stream) {
-    if (engine == LF_GEMM_AUTO && K > 0) engine = auto_engine(K);
+    if (engine == LF_GEMM_AUTO) engine = auto_engine(M, N, K);
     const bool tc = engine == LF_GEMM_TCGEN05 || engine == LF_GEMM_TCGEN05_TMA;
     if ((!tc && engine != LF_GEMM_MMA_SYNC) || M <= 0 || N <= 0 || K <= 0 || M % kBM ||
         N % kBN || K % (tc ? kTcBK : kBK) || !A || !B || !C ||

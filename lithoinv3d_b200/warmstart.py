@@ -66,17 +66,20 @@ class Network:
 
         n = X.shape[0]
         nb = n // self.batch
+        if Y.shape[0] < n or X.shape[1] != self.n_in or Y.shape[1] != self.n_out:
+            raise IndexError(f"train: X {tuple(X.shape)}, Y {tuple(Y.shape)} for {self.n_in} -> {self.n_out}")
+        X, Y = X.contiguous(), Y.contiguous()
+        torch.cuda.current_stream(X.device).synchronize()  # the network runs on a stream of its own
         losses = []
-        loss = C.c_float()
+        loss = np.zeros(nb, np.float32)
         for e in range(epochs):
-            perm = torch.as_tensor(rng.permutation(n), device=X.device)
+            rows = np.ascontiguousarray(rng.permutation(n), np.int64)
+            if nb:
+                self._err(self.lib.lf_mlp_train_rows(self.h, X.data_ptr(), Y.data_ptr(), n, rows.ctypes.data, nb,
+                                                     float(lr), loss.ctypes.data), "train_rows")
             tot = 0.0
-            for b in range(nb):
-                idx = perm[b * self.batch:(b + 1) * self.batch]
-                xb, yb = X[idx].contiguous(), Y[idx].contiguous()
-                self._err(self.lib.lf_mlp_train_step(self.h, xb.data_ptr(), yb.data_ptr(), float(lr), C.byref(loss)),
-                          "train_step")
-                tot += loss.value
+            for v in loss.tolist():
+                tot += v
             losses.append(tot / max(nb, 1))
             lr *= lr_decay
         return losses
@@ -84,8 +87,10 @@ class Network:
     def predict(self, X):
         import torch
 
+        X = X.contiguous()
         out = torch.zeros((X.shape[0], self.n_out), dtype=torch.float32, device=X.device)
-        self._err(self.lib.lf_mlp_predict(self.h, X.contiguous().data_ptr(), X.shape[0], out.data_ptr()), "predict")
+        torch.cuda.current_stream(X.device).synchronize()  # the network runs on a stream of its own
+        self._err(self.lib.lf_mlp_predict(self.h, X.data_ptr(), X.shape[0], out.data_ptr()), "predict")
         return out
 
     def predict_one(self, feat: np.ndarray) -> np.ndarray:
