@@ -41,6 +41,16 @@ struct MmaShape {
     static constexpr int kSmem = kRing * 2;            // bytes
 };
 
+// A kernel launched with programmatic stream serialisation (launch_next) may
+// be put on the SMs before the kernels ahead of it in the stream are done.
+// Every kernel of the training chain calls this before its first access to
+// memory: it lets the next one on in turn, and waits until the work ahead is
+// complete and visible.  Without that launch attribute it does nothing.
+__device__ __forceinline__ void wait_for_stream() {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+}
+
 enum Epilogue {
     EPI_F32 = 0,        // C fp32
     EPI_BIAS_RELU = 1,  // bf16 relu(C + bias[n])
@@ -191,6 +201,7 @@ __global__ void __launch_bounds__(MmaShape<BT>::kThreads)
                 const __nv_bfloat16* __restrict__ y) {
     using Sh = MmaShape<BT>;
     extern __shared__ __align__(16) __nv_bfloat16 ring[];
+    wait_for_stream();
     const int m0 = blockIdx.y * BT, n0 = blockIdx.x * BT;
     float acc[Sh::kMI][Sh::kNI][4];
     mma_tile_sum<BT, A_T, B_T>(acc, ring, K / Sh::kBK, A, lda, m0, B, ldb, n0);
@@ -221,6 +232,7 @@ __global__ void __launch_bounds__(MmaShape<BT>::kThreads)
 // boundary.
 __global__ void k_load_input(int n_rows, int batch, int n, int n_pad, bool vec, const float* __restrict__ x,
                              const long long* __restrict__ rows, __nv_bfloat16* __restrict__ y) {
+    wait_for_stream();
     const size_t i = 4 * (blockIdx.x * (size_t)blockDim.x + threadIdx.x);
     if (i >= (size_t)batch * n_pad) return;
     const int r = (int)(i / n_pad), c = (int)(i % n_pad);
@@ -247,6 +259,7 @@ __global__ void k_load_input(int n_rows, int batch, int n, int n_pad, bool vec, 
 // r's target is row target_rows[r], or r itself.
 __global__ void k_mse(int rows, int cols, int n_valid, const float* __restrict__ pred, const float* __restrict__ target,
                       const long long* __restrict__ target_rows, int ld_target, __nv_bfloat16* __restrict__ dpred, float* __restrict__ block_loss) {
+    wait_for_stream();
     __shared__ float red[256];
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const float inv = 1.f / ((float)rows * (float)n_valid);
@@ -357,6 +370,7 @@ template <bool UPDATE>
 __global__ void __launch_bounds__(MmaShape<64>::kThreads) k_layer_grads(const __grid_constant__ LayerGrads L, int batch, Adam k) {
     using Sh = MmaShape<64>;
     __shared__ __align__(16) __nv_bfloat16 ring[Sh::kRing];
+    wait_for_stream();
     int l = 0;
     while (l + 1 < L.n && (int)blockIdx.x >= L.layer[l + 1].block0) ++l;
     const LayerGrad& g = L.layer[l];
