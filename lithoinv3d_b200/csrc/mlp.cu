@@ -15,6 +15,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <random>
@@ -221,12 +222,15 @@ static cudaError_t launch_mma(cudaStream_t stream, int M, int N, int K, const __
                               const __nv_bfloat16* B, int ldb, const float* bias, float* Cf, __nv_bfloat16* Cb,
                               int ldc, const __nv_bfloat16* y) {
     using Sh = MmaShape<BT>;
-    static bool attr = false;  // per instantiation, per process
-    if (Sh::kSmem > 48 * 1024 && !attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_bf16<BT, A_T, B_T, EPI>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem);
+    if (Sh::kSmem > 48 * 1024) {
+        static std::atomic<unsigned long long> allowed{0};  // per instantiation: the devices it is set on
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess && (dev >= 64 || !(allowed.load() >> dev & 1)))
+            e = cudaFuncSetAttribute(k_gemm_bf16<BT, A_T, B_T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     Sh::kSmem);
         if (e != cudaSuccess) return e;
-        attr = true;
+        if (dev < 64) allowed.fetch_or(1ull << dev);
     }
     return launch_next(k_gemm_bf16<BT, A_T, B_T, EPI>, dim3(N / BT, M / BT), Sh::kThreads, Sh::kSmem, stream, K, A, lda,
                        B, ldb, bias, Cf, Cb, ldc, y);
@@ -441,8 +445,8 @@ static lf_status backward(lf_mlp* m, const float* d_y, const Adam* update, const
                               L.vw.p, L.b.p, L.gb.p, L.mb.p, L.vb.p, L.wb.p, L.in, L.out, blocks};
                 blocks += (L.in / 64) * (L.out / 64) + L.out / 32;
             }
-            launch_next(update ? k_layer_grads<true> : k_layer_grads<false>, blocks, MmaShape<64>::kThreads, 0, m->stream,
-                        G, m->batch, update ? *update : Adam{});
+            launch_next(update ? k_layer_grads<true> : k_layer_grads<false>, blocks, MmaShape<64>::kThreads, 0,
+                        m->stream, G, m->batch, update ? *update : Adam{});
         }
     } else {
         for (int l = m->depth; l >= 0; --l) {

@@ -258,7 +258,8 @@ __global__ void k_load_input(int n_rows, int batch, int n, int n_pad, bool vec, 
 // gradient w.r.t. pred (bf16, padding columns zero) and per-block sums.  Row
 // r's target is row target_rows[r], or r itself.
 __global__ void k_mse(int rows, int cols, int n_valid, const float* __restrict__ pred, const float* __restrict__ target,
-                      const long long* __restrict__ target_rows, int ld_target, __nv_bfloat16* __restrict__ dpred, float* __restrict__ block_loss) {
+                      const long long* __restrict__ target_rows, int ld_target, __nv_bfloat16* __restrict__ dpred,
+                      float* __restrict__ block_loss) {
     wait_for_stream();
     __shared__ float red[256];
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -367,7 +368,8 @@ struct LayerGrads {
 };
 
 template <bool UPDATE>
-__global__ void __launch_bounds__(MmaShape<64>::kThreads) k_layer_grads(const __grid_constant__ LayerGrads L, int batch, Adam k) {
+__global__ void __launch_bounds__(MmaShape<64>::kThreads)
+    k_layer_grads(const __grid_constant__ LayerGrads L, int batch, Adam k) {
     using Sh = MmaShape<64>;
     __shared__ __align__(16) __nv_bfloat16 ring[Sh::kRing];
     wait_for_stream();
