@@ -468,7 +468,9 @@ template <bool GZ, bool TMI>
 __device__ __forceinline__ void pair_forward_fp64(const double* __restrict__ F, d3 o, double* gz, double* tmi) {
     const double2* __restrict__ q = reinterpret_cast<const double2*>(F);
     const double2 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4];
-    if (__double2hiint(q4.y) < 0) return;  // contributes nothing (the same for every lane)
+    // contributes nothing (the same for every lane): -1 itself, since the area of
+    // a facet that overflows is a NaN with a sign bit and has to reach the sums
+    if (__double2hiint(q4.y) == (int)0xbff00000) return;
     const d3 ra = mk3(q0.x - o.x, q0.y - o.y, q1.x - o.z), rb = mk3(q1.y - o.x, q2.x - o.y, q2.y - o.z),
              rc = mk3(q3.x - o.x, q3.y - o.y, q4.x - o.z);
     const double a2 = dot3(ra, ra), b2 = dot3(rb, rb), c2 = dot3(rc, rc);
