@@ -408,6 +408,14 @@ __device__ __forceinline__ double atan_poly64(double t) {
     return fma(p * w, t, t);
 }
 
+// The largest of three edge ratios v = L / (d1 + d2) by their high words.  As
+// unsigned numbers the high words of positive doubles keep their order, and a
+// NaN of either sign (a station on a vertex: its distance is 0 x inf) exceeds
+// every finite value.
+__device__ __forceinline__ unsigned max_ratio_hi(double v0, double v1, double v2) {
+    return max((unsigned)__double2hiint(v0), max((unsigned)__double2hiint(v1), (unsigned)__double2hiint(v2)));
+}
+
 // One pair (station o, facet record F) with every branch of the reference
 // (solidAngle, lineIntegralTerm) and the library functions: the gz facet
 // factor and the TMI facet factor.  Up to the logarithms and the arctangent
@@ -457,8 +465,8 @@ __device__ __noinline__ double2 pair_forward_fp64_branches(const double* __restr
 // 2.5 la lb lc and its tangent at most 0.283) and the station lies further
 // than 2^-20 la from the facet's plane (so it is on no edge's line, where the
 // reference's lineIntegralTerm is 0); every other pair, zero distances and
-// NaN among them, takes the branches above.  Both tests compare the high
-// words of positive doubles.
+// NaN among them (max_ratio_hi), takes the branches above.  Both tests compare
+// the high words of doubles.
 // Bound by the FP64 pipe: about 140 FP64 instructions per pair, against more
 // than 500 through the library functions.  Its error against 64-bit sums in
 // the symmetric form fell with the cancellation in s + d: 1.7e-13 to 2e-15 on
@@ -478,8 +486,8 @@ __device__ __forceinline__ void pair_forward_fp64(const double* __restrict__ F, 
     const double2 q5 = q[5], q6 = q[6], q7 = q[7], q8 = q[8], q9 = q[9];
     const double h = ra.x * q5.x + ra.y * q5.y + ra.z * q6.x;
     const double v0 = q7.x * rcp_pos64(la + lb), v1 = q7.y * rcp_pos64(lb + lc), v2 = q8.x * rcp_pos64(lc + la);
-    const int vmax = max(__double2hiint(v0), max(__double2hiint(v1), __double2hiint(v2)));
-    if (!(vmax < 0x3fe00000 && (__double2hiint(h) & 0x7fffffff) + (20 << 20) > __double2hiint(la))) {
+    const unsigned vmax = max_ratio_hi(v0, v1, v2);
+    if (!(vmax < 0x3fe00000u && (__double2hiint(h) & 0x7fffffff) + (20 << 20) > __double2hiint(la))) {
         const double2 r = pair_forward_fp64_branches<GZ, TMI>(F, o);
         if (GZ) *gz += r.x;
         if (TMI) *tmi += r.y;
@@ -490,7 +498,7 @@ __device__ __forceinline__ void pair_forward_fp64(const double* __restrict__ F, 
     const double den = fma(la * lb, lc, fma(dab, lc, fma(dac, lb, dbc * la)));
     const double om = atan_poly64(h * q4.y * rcp_pos64(den));
     double l0, l1, l2;
-    if (vmax < 0x3fd00000) {  // every v < 1/4
+    if (vmax < 0x3fd00000u) {  // every v < 1/4
         l0 = atanh_short64(v0);
         l1 = atanh_short64(v1);
         l2 = atanh_short64(v2);
@@ -948,10 +956,10 @@ __device__ __forceinline__ void pair_gradient_fp64(const double* C, double gsn, 
         v1 = fma(fma(-v1, D1, L1), q1, v1);
         v2 = fma(fma(-v2, D2, L2), q2, v2);
     }
-    const int vmax = max(__double2hiint(v0), max(__double2hiint(v1), __double2hiint(v2)));
+    const unsigned vmax = max_ratio_hi(v0, v1, v2);
     double om, l0, l1, l2, W0, W1, W2;
     bool lv0 = true, lv1 = true, lv2 = true;
-    if (vmax < 0x3fe00000) {  // every v < 1/2
+    if (vmax < 0x3fe00000u) {  // every v < 1/2
         W0 = (L0 + L0) * rcp_pos64(m0);
         W1 = (L1 + L1) * rcp_pos64(m1);
         W2 = (L2 + L2) * rcp_pos64(m2);
@@ -960,7 +968,7 @@ __device__ __forceinline__ void pair_gradient_fp64(const double* C, double gsn, 
                      dac = 0.5 * fma(-L2, L2, c2 + a2);
         const double den = fma(la * lb, lc, fma(dab, lc, fma(dac, lb, dbc * la)));
         om = 2.0 * atan_poly64(-z * (L0 * cy) * rcp_pos64(den));
-        if (vmax < 0x3fd00000) {  // every v < 1/4
+        if (vmax < 0x3fd00000u) {  // every v < 1/4
             l0 = 2.0 * atanh_short64(v0);
             l1 = 2.0 * atanh_short64(v1);
             l2 = 2.0 * atanh_short64(v2);

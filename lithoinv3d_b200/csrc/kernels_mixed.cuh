@@ -186,7 +186,7 @@ __device__ __forceinline__ void pair_near_f64(const double* __restrict__ s, d3 o
     const double a2 = fma(x, x, yz2), b2 = fma(rbx, rbx, yz2), c2 = fma(rcx, rcx, fma(rcy, rcy, z2));
     const double la = sqrt_pos64(a2), lb = sqrt_pos64(b2), lc = sqrt_pos64(c2);
     const double v0 = L0 * rcp_pos64(la + lb), v1 = L1 * rcp_pos64(lb + lc), v2 = L2 * rcp_pos64(lc + la);
-    if (!(max(__double2hiint(v0), max(__double2hiint(v1), __double2hiint(v2))) < 0x3fe00000)) {
+    if (!(max_ratio_hi(v0, v1, v2) < 0x3fe00000u)) {
         const double2 r = pair_near_f64_close(s, x, y, z);
         *gz += r.x;
         *tmi += r.y;
