@@ -2950,9 +2950,10 @@ extern "C" lf_status lf_constraint_penalty(lf_ctx* c, const double* params, doub
 // the scatter's tables.  A parameter that moves more than kSweepMaxVerts
 // vertices (a control point that drives most of a mesh) gets no list and is
 // evaluated by whole passes.  A model whose tables do not meet the sweep's
-// assumptions (a row that reads a row, a vertex in two averaging groups), whose
-// lists are too long, or with more than kSweepMostWhole such parameters keeps
-// the sequential sweep.
+// assumptions (a row that reads a row, a vertex in two averaging groups, two
+// parameters that write one coordinate, where the scatter's own order decides),
+// whose lists are too long, or with more than kSweepMostWhole such parameters
+// keeps the sequential sweep.
 static lf_status sweep_tables(lf_ctx* c) {
     if (c->sweepState != 0) return LF_OK;
     const int V = c->V, T = c->T, np = c->np;
@@ -2970,6 +2971,9 @@ static lf_status sweep_tables(lf_ctx* c) {
     LF_TRY_CUDA(c, fetch(adjOff, c->d_adjOff, V + 1));
     LF_TRY_CUDA(c, cudaStreamSynchronize(c->stream));
     LF_TRY_CUDA(c, fetch(refV, c->d_refVertex, dofOff[np]));
+    std::vector<uint8_t> refA(dofOff[np]);
+    if (!refA.empty())
+        LF_TRY_CUDA(c, cudaMemcpyAsync(refA.data(), c->d_refAxis.p, refA.size(), cudaMemcpyDeviceToHost, c->stream));
     LF_TRY_CUDA(c, fetch(syV, c->d_syncVertex, c->nSync ? syOff[c->nSync] : 0));
     LF_TRY_CUDA(c, fetch(rowSrc, c->d_interpSrc, c->nInterpRows ? rowOff[V] : 0));
     LF_TRY_CUDA(c, fetch(adjRow, c->d_adjRow, adjOff[V]));
@@ -2978,6 +2982,13 @@ static lf_status sweep_tables(lf_ctx* c) {
     auto isRow = [&](int v) { return c->nInterpRows && rowOff[v + 1] > rowOff[v]; };
     for (int32_t q : rowSrc)
         if (isRow(q)) return LF_OK;
+    std::vector<int32_t> writer(3 * (size_t)V, -1);
+    for (int j = 0; j < np; ++j)
+        for (int r = dofOff[j]; r < dofOff[j + 1]; ++r) {
+            int32_t& w = writer[3 * (size_t)refV[r] + refA[r]];
+            if (w >= 0 && w != j) return LF_OK;
+            w = j;
+        }
     std::vector<int32_t> sync(V, -1);
     for (int g = 0; g < c->nSync; ++g) {
         if (syOff[g + 1] - syOff[g] < 2) continue;  // k_sync_shared leaves it alone

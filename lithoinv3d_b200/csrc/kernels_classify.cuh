@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(kSweepThreads) k_constraint_sweep(SweepTables 
     const int j = blockIdx.x, minus = blockIdx.y;
     const double up = __dadd_rn(p0[j], h), val = minus ? __dsub_rn(up, __dmul_rn(2.0, h)) : up;  // as k_constraint_step
     const int rb = t.dof_off[j], re = t.dof_off[j + 1];
-    auto source = [&](int v, int axis) {
-        for (int r = rb; r < re; ++r)
+    auto source = [&](int v, int axis) {  // the last write counts, as in k_scatter_dofs
+        for (int r = re - 1; r >= rb; --r)
             if (t.ref_vertex[r] == v && t.ref_axis[r] == axis) return __dmul_rn(val, t.ref_scale[r]);
         return t.S[3 * (size_t)v + axis];
     };

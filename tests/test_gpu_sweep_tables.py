@@ -1,0 +1,82 @@
+"""The side-by-side constraint sweep on tables that the model builder does not
+make but lf_set_model_tables accepts, against a penalty evaluation at every
+perturbed parameter vector (decisions and a fixed summation order: compared
+exactly)."""
+import numpy as np
+import pytest
+
+from lithoinv3d_b200 import Context, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def context(V, F, dof_off, ref_vertex, ref_axis, ref_scale):
+    """One group's raw tables in a stateless context."""
+    ctx = Context()
+    one, zero = np.array([0.3]), np.zeros(3)
+
+    def d(a):
+        return np.ascontiguousarray(a, np.float64).ctypes.data_as(ctx.lib.lf_set_model_tables.argtypes[2])
+
+    def i(a):
+        return np.ascontiguousarray(a, np.int32).ctypes.data_as(ctx.lib.lf_set_model_tables.argtypes[11])
+
+    axis = np.ascontiguousarray(ref_axis, np.uint8)
+    st = ctx.lib.lf_set_model_tables(ctx.h, 1, d(one), d(zero), d(zero), d(zero), d(zero), d(zero), len(V), d(V),
+                                     len(F), i(F), i([0, len(F)]), len(dof_off) - 1, i(dof_off), i(ref_vertex),
+                                     axis.ctypes.data_as(ctx.lib.lf_set_model_tables.argtypes[16]), d(ref_scale),
+                                     None, None, None, 0, None, None)
+    ctx._check(st, "set_model_tables")
+    ctx.n_dofs, ctx.n_groups = len(dof_off) - 1, 1
+    ctx.set_field(60.0, 10.0, 55000.0)
+    ctx.set_gravity_data(np.array([[0.0, 0.0, 1.0]]))
+    ctx.set_scatter_stateless(True)
+    return ctx
+
+
+def intervals(ctx, points):
+    half = np.linspace(0.5, 9.0, len(points))
+    ctx.set_constraints(points[:, :2], -points[:, 2] - half, -points[:, 2] + half, np.zeros(len(points)), weight=2.5)
+
+
+def expected(ctx, x):
+    g = np.zeros(len(x))
+    for j in range(len(x)):
+        p = x.copy()
+        p[j] = x[j] + 1.0
+        fp = ctx.constraint_penalty(p)
+        p[j] = p[j] - 2.0
+        g[j] = 2.5 * ((fp - ctx.constraint_penalty(p)) / 2.0)
+    return g
+
+
+def body():
+    U, F = synth.icosphere(2)
+    return U * 200.0 + [0.0, 0.0, -500.0], F
+
+
+def test_parameter_that_writes_a_coordinate_twice():
+    """z of every vertex twice, scaled by 0.5 and then by 1: the scatter's last
+    write is the one that counts, on both sides of every step."""
+    V, F = body()
+    n = len(V)
+    ctx = context(V, F, 2 * np.arange(n + 1), np.repeat(np.arange(n), 2), np.full(2 * n, 2), np.tile([0.5, 1.0], n))
+    rng = np.random.default_rng(4)
+    intervals(ctx, V[rng.integers(0, n, 50)] + rng.uniform(-0.6, 0.6, (50, 3)))
+    x = V[:, 2].copy()
+    want = expected(ctx, x)
+    assert np.count_nonzero(want) > 0
+    assert np.array_equal(ctx.constraint_gradient(x), want)
+
+
+def test_two_parameters_on_one_coordinate():
+    """Which of the two writes stays is the scatter's affair: such tables run
+    pass by pass (at least a step and a scatter for each of the 2 np passes)."""
+    V, F = body()
+    n = len(V)
+    vertex = np.concatenate([np.arange(n), [7]])
+    ctx = context(V, F, np.arange(n + 2), vertex, np.full(n + 1, 2), np.ones(n + 1))
+    intervals(ctx, V[:20] + 0.4)
+    before = ctx.counters().launches
+    ctx.constraint_gradient(V[vertex, 2])
+    assert ctx.counters().launches - before >= 4 * (n + 1)
