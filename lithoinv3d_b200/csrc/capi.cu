@@ -2948,8 +2948,8 @@ extern "C" lf_status lf_constraint_penalty(lf_ctx* c, const double* params, doub
 
 // Vertices and triangles that each parameter moves (k_constraint_sweep), from
 // the scatter's tables.  A parameter that moves more than kSweepMaxVerts
-// vertices (a control point that drives most of a mesh) gets no list and is
-// evaluated by whole passes.  A model whose tables do not meet the sweep's
+// vertices (a control point that drives most of a mesh) or kSweepMaxTriangles
+// triangles gets no list and is evaluated by whole passes.  A model whose tables do not meet the sweep's
 // assumptions (a row that reads a row, a vertex in two averaging groups, two
 // parameters that write one coordinate, where the scatter's own order decides),
 // whose lists are too long, or with more than kSweepMostWhole such parameters
@@ -3026,24 +3026,28 @@ static lf_status sweep_tables(lf_ctx* c) {
             addWithGroup(refV[r]);
             for (int k = adjOff[refV[r]]; k < adjOff[refV[r] + 1]; ++k) addWithGroup(adjRow[k]);
         }
-        if (av.size() - first > (size_t)kSweepMaxVerts) {
-            for (size_t i = first; i < av.size(); ++i) slot[av[i]] = -1;
+        const size_t firstTri = at.size();
+        bool whole = av.size() - first > (size_t)kSweepMaxVerts;
+        for (size_t i = first; i < av.size() && !whole; ++i) {
+            for (int k = vfOff[av[i]]; k < vfOff[av[i] + 1]; ++k) {
+                const int f = vf[k] / 3;
+                if (seen[f] == j) continue;
+                seen[f] = j;
+                auto code = [&](int q) { const int v = tri[3 * (size_t)f + q]; return slot[v] >= 0 ? slot[v] : ~v; };
+                at.push_back(make_int4(code(0), code(1), code(2), f));
+            }
+            whole = at.size() - firstTri > (size_t)kSweepMaxTriangles;
+        }
+        for (size_t i = first; i < av.size(); ++i) slot[av[i]] = -1;
+        if (whole) {
             av.resize(first);
+            at.resize(firstTri);
             listOf[j] = -1;
             c->sweepWhole.push_back(j);
             if (c->sweepWhole.size() > kSweepMostWhole) return LF_OK;
             continue;
         }
-        for (size_t i = first; i < av.size(); ++i)
-            for (int k = vfOff[av[i]]; k < vfOff[av[i] + 1]; ++k) {
-                const int f = vf[k] / 3;
-                if (seen[f] == l) continue;
-                seen[f] = l;
-                auto code = [&](int q) { const int v = tri[3 * (size_t)f + q]; return slot[v] >= 0 ? slot[v] : ~v; };
-                at.push_back(make_int4(code(0), code(1), code(2), f));
-            }
-        for (size_t i = first; i < av.size(); ++i) slot[av[i]] = -1;
-        if (at.size() > kMostTriangles) return LF_OK;
+        if (at.size() > kMostTriangles || av.size() > 3 * kMostTriangles) return LF_OK;
         c->sweepMaxVerts = std::max(c->sweepMaxVerts, static_cast<int>(av.size() - first));
         avOff.push_back(static_cast<int32_t>(av.size()));
         atOff.push_back(static_cast<int32_t>(at.size()));

@@ -244,6 +244,11 @@ struct SweepTables {
 
 constexpr int kSweepThreads = 256;
 constexpr int kSweepMaxVerts = 1024, kSweepMaxPoints = 2048;  // per pass, in shared memory
+// Triangles per list: more than six per vertex only where vertices of high
+// valence move (the hub of a fan), which is work for a whole pass's many CTAs.
+constexpr int kSweepMaxTriangles = 8 * kSweepMaxVerts;
+static_assert((long long)kSweepMaxTriangles * kSweepMaxPoints + kSweepThreads < (1ll << 31),
+              "the kernel numbers a list's (triangle, point) tests with an int");
 
 __global__ void __launch_bounds__(kSweepThreads) k_constraint_sweep(SweepTables t, int np, const double* __restrict__ p0,
                                                                     double h, int n, const double* __restrict__ pts,

@@ -80,3 +80,31 @@ def test_two_parameters_on_one_coordinate():
     before = ctx.counters().launches
     ctx.constraint_gradient(V[vertex, 2])
     assert ctx.counters().launches - before >= 4 * (n + 1)
+
+
+def test_lists_of_many_triangles():
+    """1,024 fans whose hubs move together: the list's triangles times the points
+    exceed 2^31, so that parameter is a whole pass; those numbered after it (a
+    rim vertex, then a hub's neighbour) keep complete lists."""
+    fans, rim, n = 1024, 1030, 2048
+    assert fans * rim * n > 2 ** 31
+    a = np.arange(rim) * (2 * np.pi / rim)
+    one = np.concatenate([[[0.0, 0.0, 0.0]], np.stack([40.0 * np.cos(a), 40.0 * np.sin(a), np.full(rim, -30.0)], 1)])
+    at = synth.station_grid(32, 100.0, -100.0)
+    V = (at[:, None] + one[None]).reshape(-1, 3)
+    k = np.arange(1, rim + 1)
+    tri = np.stack([np.zeros_like(k), k, np.roll(k, -1)], 1)
+    F = (np.arange(fans)[:, None, None] * (rim + 1) + tri[None]).reshape(-1, 3).astype(np.int32)
+    hubs = np.arange(fans) * (rim + 1)
+    moved = np.concatenate([hubs, [3], [4 * (rim + 1) + 7]])
+    ctx = context(V, F, [0, fans, fans + 1, fans + 2], moved, np.full(fans + 2, 2), np.ones(fans + 2))
+    rng = np.random.default_rng(1)
+    t, u, f = rng.uniform(0, 2 * np.pi, n), rng.uniform(0.1, 0.9, n), rng.integers(0, fans, n)
+    t[::4], u[::4], f[::4] = a[2] + 1e-4, 0.97, 0  # beside the other two parameters' vertices
+    t[1::4], u[1::4], f[1::4] = a[6] - 1e-4, 0.97, 4
+    pts = at[f] + np.stack([40.0 * u * np.cos(t), 40.0 * u * np.sin(t), -30.0 * u + rng.uniform(-0.4, 0.4, n)], 1)
+    intervals(ctx, pts)
+    x = V[moved[[0, fans, fans + 1]], 2]
+    want = expected(ctx, x)
+    assert np.all(want != 0)
+    assert np.array_equal(ctx.constraint_gradient(x), want)
