@@ -196,8 +196,11 @@ struct lf_ctx {
     DevBuf<double> d_cMid, d_cThick, d_cPar, d_cPar0, d_cFp, d_cFm, d_cGrad, d_cOut, d_pts;
     // Side-by-side sweep (k_constraint_sweep): which vertices and triangles each
     // parameter moves, built on first use.  sweepState 0: not built, 1: built,
-    // -1: the model needs the sequential sweep.
+    // 2: counted only, the sequential sweep was the faster one, -1: the model
+    // needs the sequential sweep.
     int sweepState = 0, sweepMaxVerts = 0;
+    int sweepLongest = 0;        // triangles of the longest list
+    long long sweepListed = 0;   // triangles of every parameter's list, added
     std::vector<int32_t> sweepWhole;  // parameters evaluated by whole passes
     DevBuf<int32_t> d_swList, d_swAvOff, d_swAv, d_swAtOff, d_swSync, d_swPre;
     DevBuf<int4> d_swAt;
@@ -2946,16 +2949,32 @@ extern "C" lf_status lf_constraint_penalty(lf_ctx* c, const double* params, doub
     return LF_OK;
 }
 
+// Whether the side-by-side sweep is the faster one.  Few parameters with long
+// lists under many points leave it a serial chain in a handful of CTAs, while a
+// sequential pass spreads its T x n tests over the GPU.  Estimates in
+// microseconds from times on a B200: a CTA does 250 list tests per microsecond,
+// the GPU 50,000 when full; a pass costs 22 replayed from the graph, 35
+// launched, and T x n / 180,000 for its tests.  Whole gradient, side by side
+// and sequential (parameters, facets, longest list): 16, 2,288, 948 under 64 /
+// 256 / 2,048 points 0.32 and 0.63, 0.94 and 0.80, 9.0 and 1.8 ms; 50, 12,888,
+// 2,483 under 256 / 1,024 points 2.8 and 4.3, 13.0 and 9.4 ms; 392, 44,596,
+// 2,548 under 2,048 points 34 and 432 ms.
+static bool side_by_side_is_faster(const lf_ctx* c) {
+    const double n = c->nCons, tests = c->T * n / 180000.0;
+    const double lists = std::max(c->sweepLongest * n / 250.0, 2.0 * c->sweepListed * n / 50000.0);
+    return lists + 2.0 * c->sweepWhole.size() * (35.0 + tests) <= 2.0 * c->np * (22.0 + tests);
+}
+
 // Vertices and triangles that each parameter moves (k_constraint_sweep), from
 // the scatter's tables.  A parameter that moves more than kSweepMaxVerts
 // vertices (a control point that drives most of a mesh) or kSweepMaxTriangles
-// triangles gets no list and is evaluated by whole passes.  A model whose tables do not meet the sweep's
-// assumptions (a row that reads a row, a vertex in two averaging groups, two
-// parameters that write one coordinate, where the scatter's own order decides),
-// whose lists are too long, or with more than kSweepMostWhole such parameters
-// keeps the sequential sweep.
+// triangles gets no list and is evaluated by whole passes.  A model whose
+// tables do not meet the sweep's assumptions (a row that reads a row, a vertex
+// in two averaging groups, two parameters that write one coordinate, where the
+// scatter's own order decides) or whose lists are too long together keeps the
+// sequential sweep.
 static lf_status sweep_tables(lf_ctx* c) {
-    if (c->sweepState != 0) return LF_OK;
+    if (c->sweepState == 1 || c->sweepState == -1 || (c->sweepState == 2 && !side_by_side_is_faster(c))) return LF_OK;
     const int V = c->V, T = c->T, np = c->np;
     auto fetch = [&](std::vector<int32_t>& h, const DevBuf<int32_t>& d, size_t n) {
         h.assign(n, 0);
@@ -2998,8 +3017,9 @@ static lf_status sweep_tables(lf_ctx* c) {
         }
     }
     constexpr size_t kMostTriangles = size_t(8) << 20;  // 128 MB of lists
-    constexpr size_t kSweepMostWhole = 64;
     c->sweepMaxVerts = 1;
+    c->sweepLongest = 0;
+    c->sweepListed = 0;
     c->sweepWhole.clear();
     std::vector<int32_t> listOf(np), avOff{0}, av, atOff{0}, slot(V, -1), seen(T, -1);
     std::vector<int4> at;
@@ -3008,6 +3028,7 @@ static lf_status sweep_tables(lf_ctx* c) {
         const int b = dofOff[j], n = dofOff[j + 1] - b;
         if (j > 0 && listOf[j - 1] >= 0 && n == b - dofOff[j - 1] && std::equal(r0 + b, r0 + b + n, r0 + dofOff[j - 1])) {
             listOf[j] = listOf[j - 1];  // another axis of the same vertices
+            c->sweepListed += atOff[listOf[j] + 1] - atOff[listOf[j]];
             continue;
         }
         const int l = static_cast<int>(avOff.size()) - 1;
@@ -3022,12 +3043,13 @@ static lf_status sweep_tables(lf_ctx* c) {
             if (sync[v] < 0) return add(v);
             for (int k = syOff[sync[v]]; k < syOff[sync[v] + 1]; ++k) add(syV[k]);
         };
-        for (int r = b; r < b + n; ++r) {
+        auto tooMany = [&] { return av.size() - first > (size_t)kSweepMaxVerts; };
+        for (int r = b; r < b + n && !tooMany(); ++r) {
             addWithGroup(refV[r]);
-            for (int k = adjOff[refV[r]]; k < adjOff[refV[r] + 1]; ++k) addWithGroup(adjRow[k]);
+            for (int k = adjOff[refV[r]]; k < adjOff[refV[r] + 1] && !tooMany(); ++k) addWithGroup(adjRow[k]);
         }
         const size_t firstTri = at.size();
-        bool whole = av.size() - first > (size_t)kSweepMaxVerts;
+        bool whole = tooMany();
         for (size_t i = first; i < av.size() && !whole; ++i) {
             for (int k = vfOff[av[i]]; k < vfOff[av[i] + 1]; ++k) {
                 const int f = vf[k] / 3;
@@ -3044,13 +3066,18 @@ static lf_status sweep_tables(lf_ctx* c) {
             at.resize(firstTri);
             listOf[j] = -1;
             c->sweepWhole.push_back(j);
-            if (c->sweepWhole.size() > kSweepMostWhole) return LF_OK;
             continue;
         }
         if (at.size() > kMostTriangles || av.size() > 3 * kMostTriangles) return LF_OK;
         c->sweepMaxVerts = std::max(c->sweepMaxVerts, static_cast<int>(av.size() - first));
+        c->sweepLongest = std::max(c->sweepLongest, static_cast<int>(at.size() - firstTri));
+        c->sweepListed += static_cast<long long>(at.size() - firstTri);
         avOff.push_back(static_cast<int32_t>(av.size()));
         atOff.push_back(static_cast<int32_t>(at.size()));
+    }
+    if (!side_by_side_is_faster(c)) {
+        c->sweepState = 2;
+        return LF_OK;
     }
     if (at.empty()) at.push_back(make_int4(0, 0, 0, 0));
     if (av.empty()) av.push_back(0);
@@ -3136,13 +3163,14 @@ extern "C" lf_status lf_constraint_gradient(lf_ctx* c, const double* params, dou
         LF_CHECK_LAUNCH(c);
         return LF_OK;
     };
-    // A stateless scatter makes the passes independent: all of them side by side
+    // A stateless scatter makes the passes independent: all of them side by side,
+    // where that is faster
     const bool independent =
         c->statelessScatter && c->G <= 64 && c->nCons > 0 && c->nCons <= kSweepMaxPoints && c->T > 0;
     if (independent) LF_RET_IF(sweep_tables(c));
     // graph replay up to 4096 parameters (about 66k graph nodes); beyond that
     // the capture itself would cost more than the launches it saves
-    if (independent && c->sweepState == 1)
+    if (independent && c->sweepState == 1 && side_by_side_is_faster(c))
         LF_RET_IF(sweep_side_by_side(c));
     else if (c->np <= 4096)
         LF_RET_IF(run_cached(c, c->gCons, c->d_cPar0.p, c->d_cFp.p, c->d_cGrad.p, sweep, true));

@@ -108,3 +108,58 @@ def test_lists_of_many_triangles():
     want = expected(ctx, x)
     assert np.all(want != 0)
     assert np.array_equal(ctx.constraint_gradient(x), want)
+
+
+def launches(ctx, x):
+    before = ctx.counters().launches
+    g = ctx.constraint_gradient(x)
+    return g, ctx.counters().launches - before
+
+
+@pytest.mark.parametrize("numbers", [(64, 2048), (2048, 64, 2048)])
+def test_route_of_few_long_lists(numbers):
+    """16 parameters that each move up to 381 vertices: under few points side by
+    side (fewer launches than passes), under many pass by pass (several launches
+    each on the first, direct run), with the same values, in either order."""
+    p = synth.voxel_contact_model(shape=(12, 10, 6), n_groups=2, n_side=4, cp_stride=4)
+    m = p.build_model()
+    rng = np.random.default_rng(7)
+    x = m.assemble_parameters() + rng.normal(0.0, 3.0, m.n_dofs)
+    ctx = p.make_context(m)
+    ctx.set_scatter_stateless(True)
+    ctx.forward(x)
+    pos = ctx.positions(m.info().n_vertices)
+    for n in numbers:
+        mid = pos[rng.integers(0, len(pos), n)] + rng.uniform(-0.6, 0.6, (n, 3))
+        half = rng.uniform(0.5, 9.0, n)
+        ctx.set_constraints(mid[:, :2], -mid[:, 2] - half, -mid[:, 2] + half, rng.integers(0, 2, n), weight=2.5)
+        want = expected(ctx, x)
+        assert np.count_nonzero(want) > 0
+        g, count = launches(ctx, x)
+        assert np.array_equal(g, want)
+        assert count < 2 * m.n_dofs if n == 64 else count >= 4 * 2 * m.n_dofs
+
+
+def test_many_parameters_that_move_much():
+    """70 parameters of 1,030 vertices each, which run as whole passes, do not
+    hold back the 300 others: fewer launches than two per pass."""
+    U, F = synth.icosphere(6)
+    V = U * 200.0 + [0.0, 0.0, -500.0]
+    heavy, each, light = 70, 1030, 300
+    coordinate = np.arange(heavy * each)
+    vertex = np.concatenate([coordinate % len(V), np.arange(light)])
+    axis = np.concatenate([coordinate // len(V), np.full(light, 2)])
+    off = np.concatenate([np.arange(heavy + 1) * each, heavy * each + np.arange(1, light + 1)])
+    # a heavy parameter is a factor on its coordinates, so that one number writes them all
+    scale = np.concatenate([V[vertex[:heavy * each], axis[:heavy * each]] / 1000.0, np.ones(light)])
+    ctx = context(V, F, off, vertex, axis, scale)
+    rng = np.random.default_rng(2)
+    near = rng.integers(0, len(V), 64)
+    near[::2] = rng.integers(0, light, 32)
+    intervals(ctx, V[near] + rng.uniform(-0.3, 0.3, (64, 3)))
+    x = np.concatenate([np.full(heavy, 1000.0), V[:light, 2]])
+    want = expected(ctx, x)
+    assert np.count_nonzero(want[:heavy]) > 0 and np.count_nonzero(want[heavy:]) > 0
+    g, count = launches(ctx, x)
+    assert np.array_equal(g, want)
+    assert count < 2 * 2 * len(x)
