@@ -1072,32 +1072,41 @@ constexpr int kFwdResident = 148 * 5;  // CTAs of k_forward_fp64 the GPU holds a
 // path's persistent schedule) counts as 148 x 8 there.
 static int fwd_blocks(const lf_ctx* c) { return c->tune.fwd_target_blocks > 0 ? c->tune.fwd_target_blocks : 148 * 8; }
 
-// Facet chunks for the forward: contiguous ranges inside one group, sized so
-// that station tiles x chunks fill the GPU.
-// With c->groupFilter >= 0 only that group's facets are planned (unit
-// responses).  fp64: the plan of k_forward_fp64.  Least facets per chunk: 32
-// there (9,900 facets under 2,964 stations: 330, 316, 308 us at 128, 64, 32),
-// 64 in mixed precision (two full shared-memory stages).  An FP64 launch that
-// would not fill the GPU twice over at 32 facets takes the sliced form with
-// 32 stations per CTA and 16 to 32 facets per chunk (a 320-facet body under
-// 529 stations: 30 us with 64-facet chunks and 128 stations, 11 us now; finer
-// chunks instead of slices are as fast, but their partials cost a new
+// Facets per chunk of the forward.  fp64: of k_forward_fp64.  Least facets per
+// chunk: 32 there (9,900 facets under 2,964 stations: 330, 316, 308 us at 128,
+// 64, 32), 64 in mixed precision (two full shared-memory stages).  An FP64
+// launch that would not fill the GPU twice over at 32 facets takes the sliced
+// form with 32 stations per CTA and 16 to 32 facets per chunk (a 320-facet body
+// under 529 stations: 30 us with 64-facet chunks and 128 stations, 11 us now;
+// finer chunks instead of slices are as fast, but their partials cost a new
 // context's first call another 0.3 ms of allocation).
+struct ChunkRule {
+    int slices, least, size;  // facet slices per CTA, least and planned facets per chunk
+};
+static ChunkRule chunk_rule(const lf_ctx* c, int nf, int S, bool fp64) {
+    const int sBlocks = std::max(1, cdiv(S, kFwdThreads));
+    const int want = std::max(1, cdiv(fwd_blocks(c), sBlocks));
+    ChunkRule r{1, fp64 ? 32 : 64, 0};
+    if (fp64 && (long long)sBlocks * cdiv(nf, 32) < 2 * kFwdResident) {
+        r.slices = 4;
+        r.least = std::min(32, std::max(16, cdiv((long long)nf * cdiv(S, 32), kFwdResident)));
+    }
+    r.size = std::max(r.least, cdiv(std::max(nf, 1), want));
+    return r;
+}
+
+// Facet chunks for the forward: contiguous ranges inside one group, sized so
+// that station tiles x chunks fill the GPU.  With c->groupFilter >= 0 only that
+// group's facets are planned (unit responses).
 static void plan_chunks(lf_ctx* c, int S, bool fp64) {
     const int g0 = c->groupFilter >= 0 ? c->groupFilter : 0, g1 = c->groupFilter >= 0 ? c->groupFilter + 1 : c->G;
     const int nf = c->grpTriOff[g1] - c->grpTriOff[g0];
-    int sBlocks = std::max(1, cdiv(S, kFwdThreads));
-    int want = std::max(1, cdiv(fwd_blocks(c), sBlocks));
-    int least = fp64 ? 32 : 64;
-    c->fp64Slices = 1;
-    if (fp64 && (long long)sBlocks * cdiv(nf, 32) < 2 * kFwdResident) {
-        c->fp64Slices = 4;
-        least = std::min(32, std::max(16, cdiv((long long)nf * cdiv(S, 32), kFwdResident)));
-    }
+    const ChunkRule rule = chunk_rule(c, nf, S, fp64);
+    const int least = rule.least, chunkSize = rule.size;
+    c->fp64Slices = rule.slices;
     if (c->chunkCapacityS == S && c->chunkFilter == c->groupFilter && c->chunkLeast == least && !c->chunksDirty &&
         !c->chunkBegin.empty())
         return;
-    int chunkSize = std::max(least, cdiv(std::max(nf, 1), want));
     c->chunkBegin.clear(); c->chunkEnd.clear(); c->chunkGroup.clear();
     for (int g = g0; g < g1; ++g)
         for (int f = c->grpTriOff[g]; f < c->grpTriOff[g + 1]; f += chunkSize) {
@@ -1276,22 +1285,36 @@ static lf_status forward_set(lf_ctx* c, const StationSet& s, double* d_gz, doubl
     int S = s.n;
     if (S == 0) return LF_OK;
     plan_chunks(c, S, true);
+    // Unit responses go through the groups one by one and hold one data type at
+    // a time: their buffers are sized for the largest group at once, and both
+    // types share the partials, since each growth is a cudaFree and a cudaMalloc
+    // (a new context's four columns of a two-group model under 2,520 stations
+    // 1.65 ms growing, 0.56 ms this way; later passes 0.52).
+    const bool unit = c->groupFilter >= 0;
+    DevBuf<double>& partM = unit ? c->d_partG : c->d_partM;
+    int nch = static_cast<int>(c->chunkBegin.size()), most = nch;
+    for (int g = 0; unit && g < c->G; ++g) {
+        const int nf = c->grpTriOff[g + 1] - c->grpTriOff[g];
+        most = std::max(most, cdiv(nf, chunk_rule(c, nf, S, true).size));
+    }
+    if (unit && c->chunksDirty)
+        for (DevBuf<int32_t>* b : {&c->d_chunkBegin, &c->d_chunkEnd, &c->d_chunkGroup})
+            LF_TRY_CUDA(c, b->reserve(most));
     lf_status st = upload_chunks(c);
     if (st != LF_OK) return st;
-    int nch = static_cast<int>(c->chunkBegin.size());
-    if (GZ) LF_TRY_CUDA(c, c->d_partG.reserve((size_t)nch * S));
-    if (TMI) LF_TRY_CUDA(c, c->d_partM.reserve((size_t)nch * S));
+    if (GZ) LF_TRY_CUDA(c, c->d_partG.reserve((size_t)most * S));
+    if (TMI) LF_TRY_CUDA(c, partM.reserve((size_t)most * S));
     if (nch > 0) {
         const bool sliced = c->fp64Slices > 1;
         const auto kernel = sliced ? k_forward_fp64<GZ, TMI, kFwdFacetTile, 4> : k_forward_fp64<GZ, TMI, kFwdFacetTile, 1>;
         int slot = prof_begin(c, c->evFwd, c->nFwd);
         kernel<<<dim3(cdiv(S, sliced ? 32 : kFwdThreads), nch), kFwdThreads, 0, c->stream>>>(
             S, s.d_xyz.p, c->d_fc.p, c->d_chunkBegin.p, c->d_chunkEnd.p, GZ ? c->d_partG.p : nullptr,
-            TMI ? c->d_partM.p : nullptr);
+            TMI ? partM.p : nullptr);
         prof_end(c, c->evFwd, slot);
     }
     k_forward_reduce<<<cdiv(S, 32), 256, 0, c->stream>>>(S, nch, c->d_chunkGroup.p, c->d_groups.p,
-                                                          GZ ? c->d_partG.p : nullptr, TMI ? c->d_partM.p : nullptr,
+                                                          GZ ? c->d_partG.p : nullptr, TMI ? partM.p : nullptr,
                                                           GZ ? d_gz : nullptr, TMI ? d_tmi : nullptr);
     c->counters.launches += 2;
     c->counters.forward_pairs += (uint64_t)S * (uint64_t)c->chunkFacets;
