@@ -8,6 +8,7 @@
 #include "lbfgsb.hpp"
 #include "model_builder.hpp"
 #include "patches.hpp"
+#include "per_device.hpp"
 
 #include <cuda_runtime.h>
 
@@ -1352,7 +1353,11 @@ static void plan_patch_chunks(lf_ctx* c, int S) {
 
 template <bool GZ, bool TMI, int NT>
 static cudaError_t patch_kernel_attrs() {
-    static const cudaError_t e = [] {
+    static PerDevice limit;  // per instantiation
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return limit.once(dev, [] {
         cudaError_t a = cudaFuncSetAttribute(k_forward_patch<GZ, TMI, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(PatchSmem<NT>));
         cudaError_t b = cudaFuncSetAttribute(k_forward_patch_items<GZ, TMI, NT>,
@@ -1360,8 +1365,7 @@ static cudaError_t patch_kernel_attrs() {
         cudaError_t d = cudaFuncSetAttribute(k_forward_patch_persistent<GZ, TMI, NT>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PatchSmem<NT>));
         return a != cudaSuccess ? a : (b != cudaSuccess ? b : d);
-    }();
-    return e;
+    });
 }
 
 // Per-evaluation records of the mixed forward: the per-facet FP64 / FP32

@@ -9,19 +9,20 @@
 // zero targets and are masked out of the loss.
 #include "../../include/litho_gpu.h"
 #include "mlp_kernels.cuh"
+#include "per_device.hpp"
 #include "tc_gemm.cuh"
 #include "tc_gemm_tma.cuh"
 
 #include <cudaTypedefs.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <random>
 #include <string>
 #include <vector>
 
+using litho_b200::PerDevice;
 using namespace litho_b200::mlp;
 
 namespace {
@@ -102,19 +103,24 @@ static lf_status mlp_check_launch(lf_mlp* m) {
     return LF_OK;
 }
 
+// Raises the kernel's dynamic shared-memory limit on the current device.
+template <typename... P>
+static cudaError_t allow_smem(PerDevice& limit, void (*kernel)(P...), int bytes) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return limit.once(dev, [&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
+}
+
 // One GEMM on `stream`: the tcgen05 kernel (K a multiple of 64; 128 x 256
 // tiles when N allows, else 128 x 128) or the warp-level mma.sync kernel
 // (K a multiple of 32).
 template <bool A_T, bool B_T, int EPI, int BN>
 static cudaError_t gemm_tc(cudaStream_t stream, int M, int N, int K, const __nv_bfloat16* A, int lda,
                            const __nv_bfloat16* B, int ldb, const float* bias, float* Cf, __nv_bfloat16* Cb, int ldc) {
-    static bool attr = false;  // per instantiation, per process (the attribute is per function)
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<A_T, B_T, EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             TcShape<BN>::kSmem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static PerDevice limit;  // per instantiation
+    const cudaError_t e = allow_smem(limit, k_gemm_tc<A_T, B_T, EPI, BN>, TcShape<BN>::kSmem);
+    if (e != cudaSuccess) return e;
     dim3 grid(N / BN, M / kBM);
     k_gemm_tc<A_T, B_T, EPI, BN><<<grid, kTcThreads, TcShape<BN>::kSmem, stream>>>(M, N, K, A, lda, B, ldb, bias, Cf,
                                                                                   Cb, ldc);
@@ -153,13 +159,9 @@ static bool bf16_map(CUtensorMap* map, const void* base, int rows, int cols, int
 template <bool A_T, bool B_T, int EPI, int BN>
 static cudaError_t gemm_tma(cudaStream_t stream, int M, int N, int K, const __nv_bfloat16* A, int lda,
                             const __nv_bfloat16* B, int ldb, const float* bias, float* Cf, __nv_bfloat16* Cb, int ldc) {
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_tma<A_T, B_T, EPI, BN>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, TmaShape<BN>::kSmem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static PerDevice limit;
+    const cudaError_t e = allow_smem(limit, k_gemm_tma<A_T, B_T, EPI, BN>, TmaShape<BN>::kSmem);
+    if (e != cudaSuccess) return e;
     CUtensorMap mapA, mapB;
     const bool okA = A_T ? bf16_map(&mapA, A, K, M, lda, 64) : bf16_map(&mapA, A, M, K, lda, kBM);
     const bool okB = B_T ? bf16_map(&mapB, B, N, K, ldb, BN) : bf16_map(&mapB, B, K, N, ldb, 64);
@@ -223,14 +225,9 @@ static cudaError_t launch_mma(cudaStream_t stream, int M, int N, int K, const __
                               int ldc, const __nv_bfloat16* y) {
     using Sh = MmaShape<BT>;
     if (Sh::kSmem > 48 * 1024) {
-        static std::atomic<unsigned long long> allowed{0};  // per instantiation: the devices it is set on
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess && (dev >= 64 || !(allowed.load() >> dev & 1)))
-            e = cudaFuncSetAttribute(k_gemm_bf16<BT, A_T, B_T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     Sh::kSmem);
+        static PerDevice limit;
+        const cudaError_t e = allow_smem(limit, k_gemm_bf16<BT, A_T, B_T, EPI>, Sh::kSmem);
         if (e != cudaSuccess) return e;
-        if (dev < 64) allowed.fetch_or(1ull << dev);
     }
     return launch_next(k_gemm_bf16<BT, A_T, B_T, EPI>, dim3(N / BT, M / BT), Sh::kThreads, Sh::kSmem, stream, K, A, lda,
                        B, ldb, bias, Cf, Cb, ldc, y);
