@@ -293,7 +293,9 @@ lf_status lf_mlp_train_step(lf_mlp* m, const float* d_x, const float* d_y, float
  * [n_rows][n_out] (device, ready on every stream): batch b takes the rows
  * rows[b * batch .. (b + 1) * batch) (host).  Same results as gathering the
  * rows and calling lf_mlp_train_step; losses[b] (host) receives batch b's
- * loss.  LF_EINVAL, with nothing trained, if a row number is out of range. */
+ * loss.  LF_EINVAL, with nothing trained, if a row number is out of range.
+ * LF_ETIMEOUT ends the call after the batch whose product gave up: that batch's
+ * loss and update are invalid, as after lf_mlp_train_step, and no later one runs. */
 lf_status lf_mlp_train_rows(lf_mlp* m, const float* d_x, const float* d_y, long long n_rows, const long long* rows,
                             int n_batches, float lr, float* losses);
 lf_status lf_mlp_predict(lf_mlp* m, const float* d_x, int rows, float* d_y);

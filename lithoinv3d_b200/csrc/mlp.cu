@@ -462,6 +462,14 @@ static lf_status backward(lf_mlp* m, const float* d_y, const Adam* update, const
     return mlp_check_launch(m);
 }
 
+// Whether no GEMM of a training step runs on the tcgen05 kernels.
+static bool trains_on_mma(const lf_mlp* m) {
+    for (const Layer& L : m->layers)
+        if (!on_mma(m, m->batch, L.out, L.in) || !on_mma(m, m->batch, L.in, L.out) || !on_mma(m, L.out, L.in, m->batch))
+            return false;
+    return true;
+}
+
 // Queues one training step.
 static lf_status queue_step(lf_mlp* m, const float* d_x, const float* d_y, const long long* d_rows, int slot,
                             float lr) {
@@ -490,8 +498,12 @@ extern "C" lf_status lf_mlp_train_rows(lf_mlp* m, const float* d_x, const float*
     for (long long i = 0; i < (long long)n_batches * m->batch; ++i)
         if (rows[i] < 0 || rows[i] >= n_rows) return LF_EINVAL;
     cudaSetDevice(m->device);
-    for (int b0 = 0; b0 < n_batches; b0 += kQueued) {
-        const int nb = std::min(kQueued, n_batches - b0);
+    // A tcgen05 product may give up on a wait: its batch is the last one then, as
+    // in single steps, so such networks are checked after every batch (their
+    // steps take far longer than the 20 us of a check).
+    const int queue = trains_on_mma(m) ? kQueued : 1;
+    for (int b0 = 0; b0 < n_batches; b0 += queue) {
+        const int nb = std::min(queue, n_batches - b0);
         const size_t n = (size_t)nb * m->batch;
         std::memcpy(m->h_rows, rows + (size_t)b0 * m->batch, sizeof(long long) * n);
         MLP_TRY(m, cudaMemcpyAsync(m->rows.p, m->h_rows, sizeof(long long) * n, cudaMemcpyHostToDevice, m->stream));
