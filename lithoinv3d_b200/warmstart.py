@@ -66,7 +66,8 @@ class Network:
 
         n = X.shape[0]
         nb = n // self.batch
-        if Y.shape[0] < n or X.shape[1] != self.n_in or Y.shape[1] != self.n_out:
+        # rows of any shape that hold n_in and n_out numbers, and no check of what no batch reads
+        if nb and (Y.shape[0] < n or X[0].numel() != self.n_in or Y[0].numel() != self.n_out):
             raise IndexError(f"train: X {tuple(X.shape)}, Y {tuple(Y.shape)} for {self.n_in} -> {self.n_out}")
         X, Y = X.contiguous(), Y.contiguous()
         torch.cuda.current_stream(X.device).synchronize()  # the network runs on a stream of its own
