@@ -1701,18 +1701,34 @@ static int grad_slots(lf_ctx* c, int S) {
     return n1;
 }
 
-// The FP32 adjoints of gradient_set's far-field kernel over S stations.
-static lf_status far_workspace(lf_ctx* c, int S) {
-    if (c->precision == LF_PREC_MIXED)
-        LF_TRY_CUDA(c, c->d_adj32.reserve(2 * (size_t)(c->partitioned ? 1 : c->G) * S));
+// Facet constants of the gradient kernels, and in mixed precision the FP32
+// adjoints of the far-field kernel for the sets whose adjoints are given.
+static lf_status grad_prep(lf_ctx* c, int want_grav, int want_mag, const double* gcoef, const double* mcoef,
+                           FarAdjoints* far) {
+    *far = FarAdjoints{};
+    if (c->precision == LF_PREC_MIXED && c->nGradFacets > 0 && (gcoef || mcoef)) {
+        far->groups = c->partitioned ? 1 : c->G;
+        far->ng = gcoef ? c->grav.n : 0;
+        far->nm = mcoef ? c->mag.n : 0;
+        far->sta_group = c->partitioned ? c->d_staGroup.p : nullptr;
+        far->gcoef = gcoef;
+        far->mcoef = mcoef;
+        LF_TRY_CUDA(c, c->d_adj32.reserve((size_t)far->count()));
+        far->out = c->d_adj32.p;
+    }
+    k_face_prep_grad<<<cdiv(c->T, kGradPrepThreads) + cdiv(far->count(), kGradPrepThreads), kGradPrepThreads, 0,
+                       c->stream>>>(c->T, c->d_tri.p, c->d_pos.p, c->d_faceGroup.p, c->d_groups.p, c->d_faceNeeds.p,
+                                    want_grav, want_mag, c->fdir, c->d_gc.p, *far);
+    LF_CHECK_LAUNCH(c);
     return LF_OK;
 }
 
-// Gradient kernels over one station set with the given adjoints (after
-// far_workspace); writes
+// Gradient kernels over one station set with the given adjoints (far: their
+// FP32 form from grad_prep); writes
 // facet partial slots [slot0, slot0 + returned count) of d_partGrad
 // ([slot][9][T], one slot per (kernel, station chunk)).
-static int gradient_set(lf_ctx* c, const StationSet& s, const double* gcoef, const double* mcoef, int slot0) {
+static int gradient_set(lf_ctx* c, const StationSet& s, const double* gcoef, const double* mcoef,
+                        const FarAdjoints& far, int slot0) {
     if (s.n == 0 || c->nGradFacets == 0) return 0;
     const bool mixed = c->precision == LF_PREC_MIXED;
     const double tau = mixed ? static_cast<double>(c->tau) : 3.0e38;
@@ -1744,11 +1760,7 @@ static int gradient_set(lf_ctx* c, const StationSet& s, const double* gcoef, con
         grad_chunks(c, s.n, false, &nch2, &tpc2);
         int ev2 = prof_begin(c, c->evGrad, c->nGrad);
         const cudaStream_t st = fork ? c->side : c->stream;
-        const int adjGroups = c->partitioned ? 1 : c->G;
-        float *adjG = c->d_adj32.p, *adjT = adjG + (size_t)adjGroups * s.n;  // reserved by far_workspace
-        k_far_adjoints<<<dim3(cdiv(s.n, 256), adjGroups), 256, 0, st>>>(
-            s.n, adjGroups, c->partitioned ? c->d_staGroup.p : nullptr, c->d_groups.p, gcoef, mcoef, adjG, adjT);
-        c->counters.launches++;
+        const float *adjG = far.out, *adjT = far.out + (size_t)far.groups * far.ng;
         const auto far32 = tau >= 3.0 ? k_gradient_warp_far32<true> : k_gradient_warp_far32<false>;
         far32<<<dim3(fblocks, nch2), 32 * kGradWarpsPerBlock, 0, st>>>(
             c->T, c->d_gc.p, s.n, s.d_xyz.p, gcoef ? adjG : nullptr, mcoef ? adjT : nullptr, s.d_tileBox.p,
@@ -1790,11 +1802,9 @@ static int gradient_fdxy_set(lf_ctx* c, const StationSet& s, const double* gcoef
 
 static lf_status gradient_all(lf_ctx* c, const double* d_params, double* d_grad) {
     bool gOn = c->grav.n > 0, mOn = c->mag.n > 0 && c->alphaMag > 0.0;
-    k_face_prep_grad<<<cdiv(c->T, 128), 128, 0, c->stream>>>(c->T, c->d_tri.p, c->d_pos.p, c->d_faceGroup.p,
-                                                             c->d_groups.p, c->d_faceNeeds.p, 1, 1, c->fdir,
-                                                             c->d_gc.p);
+    FarAdjoints far;
+    LF_RET_IF(grad_prep(c, 1, 1, gOn ? c->grav.d_coef.p : nullptr, mOn ? c->mag.d_coef.p : nullptr, &far));
     c->counters.launches++;
-    LF_CHECK_LAUNCH(c);
     int slots = 0;
     if (c->sameStations && gOn) {
         slots = grad_slots(c, c->grav.n);
@@ -1818,13 +1828,12 @@ static lf_status gradient_all(lf_ctx* c, const double* d_params, double* d_grad)
         LF_TRY_CUDA(c, cudaMemsetAsync(c->d_vgrad.p, 0, sizeof(double) * 3 * c->V, c->stream));
     } else {
         LF_TRY_CUDA(c, c->d_partGrad.reserve((size_t)slots * 9 * c->T));
-        LF_RET_IF(far_workspace(c, std::max(gOn ? c->grav.n : 0, mOn ? c->mag.n : 0)));
         int used = 0;
         if (c->sameStations && gOn) {
-            used += gradient_set(c, c->grav, c->grav.d_coef.p, mOn ? c->mag.d_coef.p : nullptr, used);
+            used += gradient_set(c, c->grav, c->grav.d_coef.p, mOn ? c->mag.d_coef.p : nullptr, far, used);
         } else {
-            if (gOn) used += gradient_set(c, c->grav, c->grav.d_coef.p, nullptr, used);
-            if (mOn) used += gradient_set(c, c->mag, nullptr, c->mag.d_coef.p, used);
+            if (gOn) used += gradient_set(c, c->grav, c->grav.d_coef.p, nullptr, far, used);
+            if (mOn) used += gradient_set(c, c->mag, nullptr, c->mag.d_coef.p, far, used);
         }
         const int fdFrom = used;
         if (fdxy) {
@@ -2325,12 +2334,11 @@ static lf_status jv_product(lf_ctx* c, StationSet& s, bool grav, const std::vect
 // w as the station coefficients, no regularisation terms.
 static lf_status jtw_product(lf_ctx* c, StationSet& s, bool grav, const std::vector<double>& w, std::vector<double>& out) {
     LF_TRY_CUDA(c, upload(c->d_tmpS, w.data(), w.size(), c->stream));
-    k_face_prep_grad<<<cdiv(c->T, 128), 128, 0, c->stream>>>(c->T, c->d_tri.p, c->d_pos.p, c->d_faceGroup.p,
-                                                             c->d_groups.p, c->d_faceNeeds.p, 1, 1, c->fdir,
-                                                             c->d_gc.p);
+    const double *gcoef = grav ? c->d_tmpS.p : nullptr, *mcoef = grav ? nullptr : c->d_tmpS.p;
+    FarAdjoints far;
+    LF_RET_IF(grad_prep(c, 1, 1, gcoef, mcoef, &far));
     LF_TRY_CUDA(c, c->d_partGrad.reserve((size_t)std::max(grad_slots(c, s.n), 1) * 9 * c->T));
-    LF_RET_IF(far_workspace(c, s.n));
-    const int used = gradient_set(c, s, grav ? c->d_tmpS.p : nullptr, grav ? nullptr : c->d_tmpS.p, 0);
+    const int used = gradient_set(c, s, gcoef, mcoef, far, 0);
     if (used > 0 && c->nGradVerts > 0)
         k_vertex_reduce<<<cdiv(c->nGradVerts, 4), 128, 0, c->stream>>>(c->nGradVerts, c->d_gradVerts.p, c->d_vfOff.p,
                                                                         c->d_vf.p, c->T, used, used, c->d_partGrad.p,
@@ -2659,10 +2667,8 @@ extern "C" lf_status lf_jacobian(lf_ctx* c, const double* params, int which, dou
     if (c->partitioned) return fail(c, LF_ESTATE, "dense Jacobian rows are not available for batched bodies");
     LF_RET_IF(params_to_device(c, params));
     LF_RET_IF(scatter(c, c->d_params.p));
-    k_face_prep_grad<<<cdiv(c->T, 128), 128, 0, c->stream>>>(c->T, c->d_tri.p, c->d_pos.p, c->d_faceGroup.p,
-                                                             c->d_groups.p, c->d_faceNeeds.p, which == LF_GRAVITY,
-                                                             which == LF_MAGNETIC, c->fdir, c->d_gc.p);
-    LF_CHECK_LAUNCH(c);
+    FarAdjoints none;
+    LF_RET_IF(grad_prep(c, which == LF_GRAVITY, which == LF_MAGNETIC, nullptr, nullptr, &none));
     int np = std::max(c->np, 1);
     // stations per batch so that the partial buffer stays below ~256 MB
     size_t per = (size_t)9 * c->T * sizeof(double);

@@ -242,22 +242,6 @@ __device__ __forceinline__ int tile_gradient_class(const FarKey& k, const double
 
 constexpr int kFarFlushTiles = 4;  // far tiles summed per lane in FP32 between warp reductions
 
-// FP32 adjoints of the far-field gradient: adjoint x group scale, rounded once
-// per (group, station) instead of once per pair.  Layout [G][S] (G = 1 with
-// every station scaled by its own body's group when sta_group is given).
-__global__ void k_far_adjoints(int S, int G, const int32_t* __restrict__ sta_group,
-                               const GroupConst* __restrict__ groups, const double* __restrict__ gcoef,
-                               const double* __restrict__ mcoef, float* __restrict__ adj_g,
-                               float* __restrict__ adj_t) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const int g = sta_group ? sta_group[s] : (int)blockIdx.y;
-    const size_t out = sta_group ? (size_t)s : (size_t)g * S + s;
-    // the scales of k_face_prep_grad (GC_GS, GC_MS)
-    if (gcoef) adj_g[out] = (float)(gcoef[s] * groups[g].gscale_jac);
-    if (mcoef) adj_t[out] = (float)(mcoef[s] * (groups[g].mag_active ? -groups[g].mscale : 0.0));
-}
-
 // Far-field objective gradient in FP32: one warp per facet, lanes over the
 // stations of the facet's far tiles (exactly the tiles k_gradient_warp_fp64
 // leaves out: both classify with facet_far_key / tile_far).  gz by Dunavant's
