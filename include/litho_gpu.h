@@ -313,8 +313,8 @@ lf_status lf_mlp_gradients(lf_mlp* m, const float* d_x, const float* d_y, float*
  *    swizzle, no multicast) in a warp-specialised pipeline (one producer
  *    warp, one MMA warp, every warp in the epilogue);
  *  LF_GEMM_AUTO (default): per GEMM, LF_GEMM_TCGEN05_TMA for a deep K on
- *    enough output tiles and LF_GEMM_MMA_SYNC otherwise (measured faster on
- *    each side of that line).
+ *    enough output tiles (K >= 2048, 48 tiles of 128 x 128) and
+ *    LF_GEMM_MMA_SYNC otherwise.
  * All give the same results to FP32 summation order. */
 enum { LF_GEMM_TCGEN05 = 0, LF_GEMM_MMA_SYNC = 1, LF_GEMM_TCGEN05_TMA = 2, LF_GEMM_AUTO = 3 };
 lf_status lf_mlp_set_engine(lf_mlp* m, int engine);

@@ -186,7 +186,7 @@ struct lf_ctx {
     DevBuf<double> d_smDiff, d_smVgrad, d_blockS;
 
     // workspaces
-    DevBuf<double> d_partG, d_partM, d_partGrad, d_blockG, d_blockM, d_ones, d_jac;
+    DevBuf<double> d_partG, d_partM, d_partGrad, d_blockG, d_blockM, d_jac;
 
     // point classification and the constraint penalty (lf_set_label_grid,
     // lf_set_bottom_depth, lf_set_constraints)

@@ -1,18 +1,23 @@
 // FP64 device kernels of the LithoInv hot path (sm_100a).
 //
-// Forward (station-per-thread, facets staged in shared memory): the per-pair
-// arithmetic follows faceNagyContribution / magneticFacet / solidAngle /
-// lineIntegralTerm of the reference in the same operation order
+// Forward (station per thread, facet records staged in shared memory): the
+// facet sums of faceNagyContribution / magneticFacet / solidAngle /
+// lineIntegralTerm of the reference
 // (modules/litho-forward/src/forward/gravity_forward.cpp:13-42,
 //  modules/litho-forward/src/forward/magnetic_forward.cpp:312-347,
-//  modules/litho-core/src/core/geometry.cpp:10-52); the station-independent
-// facet quantities (unit normal, edge vectors, lengths, in-plane edge normals,
-// magnetic direction products) are computed once per facet by face_prep_fwd.
+//  modules/litho-core/src/core/geometry.cpp:10-52).  Close to a facet's edges
+// and in its plane every operation is the reference's, in its order, so that
+// its branches are taken as it takes them; everywhere else the same sums in the
+// symmetric form, by polynomials.  The station-independent facet quantities
+// (unit normal, edge lengths, in-plane edge normals, magnetic direction
+// products) are computed once per facet by face_consts_fwd, in the reference's
+// operation order.
 //
-// Gradient (facet-per-thread, stations staged in shared memory): the
-// derivative of every facet term with respect to its three vertices, in
-// closed form, contracted with the per-station weighted residual in the same
-// pass so the Jacobian is never stored.  Derivation (per facet, local frame
+// Gradient (objective: a warp per facet, lanes over the stations; Jacobian rows:
+// a thread per facet and station): the derivative of every facet term with
+// respect to its three vertices, in closed form, contracted with the
+// per-station weighted residual in the same pass so the Jacobian is never
+// stored.  Derivation (per facet, local frame
 // with origin at vertex a, x along a->b, z along the unit normal):
 //   d Lambda_e / d p2 = ( e_hat - q W ) / d2,   d Lambda_e / d p1 = (-e_hat - q W) / d1,
 //   d Omega / d p1 += (e_hat x r1) W / d1,      d Omega / d p2 += (e_hat x r1) W / d2,
@@ -105,8 +110,9 @@ __device__ __forceinline__ double lambda_from(double s1, double s2, double d1, d
 // an exact 0 in the reference's global coordinates) -- this is the
 // continuous value log(d1 / d2) instead: the reference's forward is
 // discontinuous there and its own finite-difference Jacobian undefined.
-// The FP64 forward keeps lambda_from, bit for bit.  live = the station is
-// not on the segment itself (d1 + d2 > L).
+// The FP64 forward keeps lambda_from wherever a station may be on an edge's
+// line (pair_forward_fp64_branches).  live = the station is not on the segment
+// itself (d1 + d2 > L).
 __device__ __forceinline__ double lambda_sym(double d1, double d2, double L, bool* live) {
     const double dsum = d1 + d2, den = dsum - L;
     *live = den > 1e-13 * dsum;
@@ -254,8 +260,8 @@ __global__ void k_face_prep_fwd(int T, const int32_t* __restrict__ tri, const do
 // reference differentiates every axis by per-facet forward differences with
 // h = 1e-4 m, faceNagyWithGradient gravity_forward.cpp:48-85): forward
 // constants of each listed facet and of its six copies with one vertex moved
-// by +h in x or y, variant k = 1 + 2 * corner + axis.  Layout
-// [7][NFC][nf] over the list index.
+// by +h in x or y, variant k = 1 + 2 * corner + axis.  Layout [nf][7][NFC]
+// over the list index.
 __global__ void k_face_prep_fdxy(int nf, const int32_t* __restrict__ facets, const int32_t* __restrict__ tri,
                                  const double* __restrict__ pos, const int16_t* __restrict__ face_group,
                                  const GroupConst* __restrict__ groups, d3 fdir, double h, double* __restrict__ fcfd) {
@@ -372,8 +378,7 @@ __global__ void __launch_bounds__(kGradPrepThreads)
 // measured over 2^-40..2^40) refined by one third-order step -- Halley's for
 // x^(-1/2), y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2; for 1/x, y (1 + e + e^2)
 // with e = 1 - x y.  The remaining error is rounding: at most 1 ulp for the
-// square root and the reciprocal, 2^-51.7 for the reciprocal square root
-// (measured against the correctly rounded operations, 1.5e9 arguments).  The
+// square root and the reciprocal, 2^-51.7 for the reciprocal square root.  The
 // pair kernels evaluate seven of them per pair; the library forms cost 2-4
 // times the instructions and a special-case branch each.
 __device__ __forceinline__ double sqrt_pos64(double x) {
@@ -401,8 +406,9 @@ __device__ __forceinline__ double sqrt_inv64(double x, double* inv) {
 // atanh(v) for 0 <= v <= 1/2 (atanh_poly64), for v <= 1/4 (atanh_short64), and
 // atan(t) for t^2 <= 0.1: polynomials in the square, Chebyshev interpolants of
 // atanh(sqrt w) / sqrt w on [0, 1/4] and [0, 1/16] and of atan(sqrt w) /
-// sqrt w on [0, 0.1] (60-digit arithmetic; relative errors below 1.2e-16,
-// 9e-18 and 6e-18 before rounding).
+// sqrt w on [0, 0.1] (60-digit arithmetic; relative errors of the coefficients
+// as rounded below 1.9e-16, 1.7e-17 and 1.2e-17 before the evaluation's own
+// rounding).
 __device__ __forceinline__ double atanh_poly64(double v) {
     const double w = v * v;
     double p = fma(0.2113466728500407, w, -0.11607286571460644);
@@ -1227,8 +1233,7 @@ __global__ void __launch_bounds__(128, 3) k_gradient_warp_fp64(int T, const doub
 // Finite-difference-XY partials (see k_face_prep_fdxy): one warp per listed
 // facet x station chunk (tiles_per_chunk tiles of kStationTile stations),
 // lanes over the chunk's stations.  Per station, the facet term of the base
-// record and of the six moved copies (pair_forward_fp64, the reference's
-// operation order), contracted with the station adjoints and the group
+// record and of the six moved copies (pair_forward_fp64), contracted with the station adjoints and the group
 // scales of the analytic kernels (zero for collapsed facets):
 //   sum_s (G_s (F_k - F_0) + T_s (M_k - M_0)) / h.
 // Writes the x and y partials of the three corners, and zero z, into this

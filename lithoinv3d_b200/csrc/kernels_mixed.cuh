@@ -8,8 +8,8 @@
 //  * a facet far from a station tile (centroid distance >= tau x facet size)
 //    is integrated directly: gz facet = n_z * integral of 1/r over the facet,
 //    evaluated by quadrature in FP32 (positive terms, no cancellation):
-//    Dunavant's 6-point degree-4 rule in the forward (3 points beyond
-//    4 tau), Radon's 7-point degree-5 rule in the gradient;
+//    Dunavant's 6-point degree-4 rule, 3 points beyond 4 tau, in the forward
+//    and in the gradient;
 //  * a facet near the tile uses the analytic formula in FP64, in the facet's
 //    local frame (origin at a vertex, x along the longest edge, z along the
 //    unit normal).
@@ -40,17 +40,10 @@ enum MixedConst {
     NMC
 };
 
-// Radon's 7-point degree-5 rule on the triangle: barycentric (beta_b, beta_c)
-// of each point and its weight (weights sum to 1; multiply by the area).
-// Points: centroid; (a1,b1,b1) perms with b1 = (6 - sqrt 15)/21, a1 = 1 - 2 b1,
-// weight (155 - sqrt 15)/1200; (a2,b2,b2) perms with b2 = (6 + sqrt 15)/21,
-// weight (155 + sqrt 15)/1200; the centroid weighs 9/40.
-__constant__ float kRadonBb[7] = {0.3333333333333333f, 0.1012865073234563f, 0.7974269853530873f,
-                                  0.1012865073234563f, 0.4701420641051151f, 0.0597158717897698f,
-                                  0.4701420641051151f};
-__constant__ float kRadonBc[7] = {0.3333333333333333f, 0.1012865073234563f, 0.1012865073234563f,
-                                  0.7974269853530873f, 0.4701420641051151f, 0.4701420641051151f,
-                                  0.0597158717897698f};
+// Weights of Radon's 7-point degree-5 rule on the triangle (they sum to 1;
+// multiply by the area): 9/40 at the centroid, (155 - sqrt 15)/1200 at the
+// (a1, b1, b1) permutations with b1 = (6 - sqrt 15)/21, a1 = 1 - 2 b1, and
+// (155 + sqrt 15)/1200 at the (a2, b2, b2) ones with b2 = (6 + sqrt 15)/21.
 __constant__ float kRadonW[7] = {0.225f, 0.1259391805448271f, 0.1259391805448271f, 0.1259391805448271f,
                                  0.1323941527885062f, 0.1323941527885062f, 0.1323941527885062f};
 
@@ -333,7 +326,8 @@ __global__ void __launch_bounds__(128, 4) k_gradient_warp_far32(
             const float2 zero = make_float2(0.f, 0.f);
             float q0 = 0.f;
             float2 dqx[3], dqy[3], dqz[3];
-            // (b, c) from the first corners of edges 1 and 2, (c, a) from their second corners
+            // bc.x, bc.y: sums of vertices b and c; ca.y: of a.  ca.x stays zero: it pads the
+            // flush, where c's sum is bc.y + ca.x
             float2 bcx = zero, bcy = zero, bcz = zero, cax = zero, cay = zero, caz = zero;
             float2 am01 = zero, am2f = zero;  // sums of Ts Lambda_{0,1} / 2; Ts Lambda_2 / 2, Ts Omega / 2
 #pragma unroll

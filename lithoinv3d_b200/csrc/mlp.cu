@@ -179,8 +179,10 @@ static cudaError_t gemm_tma(cudaStream_t stream, int M, int N, int K, const __nv
 // Measured on B200, microseconds of a blocking call (20 of them its own),
 // mma.sync against tcgen05: 256 x 512 x 8192 39 / 90, 512 x 1024 x 8192
 // 79 / 91, 768 x 1024 x 8192 111 / 91, 2048 x 2048 x 8192 295 / 97; at K = 2048
-// 256 x 512 22 / 54, 1024 x 1024 41 / 54, 2048 x 2048 88 / 56.  Below K = 2048
-// tcgen05 stays behind (14.0 against 8.9 TFLOP/s at K = 512).
+// 256 x 512 22 / 54, 1024 x 1024 41 / 54, 2048 x 2048 88 / 56.  The line is that
+// of K = 8192; at K = 2048 the sizes cross between 64 and 256 tiles, so the
+// least of the products it sends to tcgen05 there are faster on mma.sync.  Below
+// K = 2048 tcgen05 stays behind (14.0 against 8.9 TFLOP/s at K = 512).
 constexpr int kAutoTmaMinK = 2048, kAutoTmaMinTiles = 48;
 static int auto_engine(int M, int N, int K) {
     const bool tma = K >= kAutoTmaMinK && K % kTcBK == 0 && (long long)(M / kBM) * (N / kBN) >= kAutoTmaMinTiles;
