@@ -463,8 +463,8 @@ __device__ __forceinline__ void forward_mixed_block(FaceF32* __restrict__ smf, d
     }
 }
 
-// Issue slots 74 % busy, special-function pipe 70 % (three to six rsqrt, three
-// rsqrt and four reciprocals, four FP64-to-FP32 conversions a pair): 147 warp
+// Issue slots 74 % busy, special-function pipe 71 % (three to six rsqrt, three
+// rsqrt and four reciprocals, four FP64-to-FP32 conversions a pair): 142 warp
 // instructions per 32 pairs with the points, vertices and series in pairs
 // (162 one by one).  19,076 facets x 4,096 stations: 460 us one by one with
 // library near pairs, 424 us now.  Seven CTAs per SM (72 registers): six

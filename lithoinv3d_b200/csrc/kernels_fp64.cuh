@@ -507,8 +507,8 @@ __device__ __noinline__ double2 pair_forward_fp64_branches(const double* __restr
 // reference's lineIntegralTerm is 0); every other pair, zero distances and
 // NaN among them (max_ratio_hi), takes the branches above.  Both tests compare
 // the high words of doubles.
-// Bound by the FP64 pipe: about 140 FP64 instructions per pair, against more
-// than 500 through the library functions.  Its error against 64-bit sums in
+// Bound by the FP64 pipe (73 % busy): 130 FP64 instructions of 227 per pair,
+// against more than 500 through the library functions.  Its error against 64-bit sums in
 // the symmetric form fell with the cancellation in s + d: 1.7e-13 to 2e-15 on
 // a 320-facet body, 1.6e-13 to 3e-15 on a contact model's unit responses.
 // The shorter atanh polynomial for v < 1/4 is worth 4 % (304 against 316 us).
@@ -606,7 +606,7 @@ __device__ __forceinline__ void forward_fp64_block(double* __restrict__ sm, int 
     }
 }
 
-// 29.6 M pairs (9,900 facets, 2,964 stations, gz and TMI): 993 us with the
+// 29.4 M pairs (9,904 facets, 2,964 stations, gz and TMI): 993 us with the
 // library functions and SoA records in shared memory, 291 us now, 1.0e11
 // pairs/s.  Five CTAs per SM: six or seven (84, 72 registers) are 3 and 6 %
 // slower, the unbounded 96 registers 2 %.
@@ -1158,9 +1158,9 @@ __device__ __forceinline__ void grad_acc_warp_sum(GradAcc& A, double* row) {
 // Warps run over `facets` (those with a DOF vertex); grid.y splits the
 // station tiles into chunks of tiles_per_chunk so that a model with few such
 // facets still fills the GPU.  part layout [chunk][9][T].
-// FP64 pipe 65 % busy at 12 warps per SM (168 registers, of which 56 hold the
+// FP64 pipe 63 % busy at 12 warps per SM (168 registers, of which 56 hold the
 // sums): 24.6 M pairs (8,308 facets, 2,964 stations) took 1,131 us with the
-// library functions, 480 us now; a 1,280-facet body under 1,600 stations 115
+// library functions, 484 us now; a 1,280-facet body under 1,600 stations 115
 // and 55 us.  Two CTAs per SM (no spill) 523 us, four (128 registers) 539;
 // CTAs of one or two warps no different.
 template <bool GZ, bool TMI>

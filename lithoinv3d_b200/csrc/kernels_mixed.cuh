@@ -259,13 +259,14 @@ constexpr int kFarFlushTiles = 4;  // far tiles summed per lane in FP32 between 
 // 4 tau x size (the omitted terms are below 2e-12), through the ninth nearer,
 // and through the thirteenth for the few pairs with an e above 0.2.
 //
-// Bound by instruction issue.  The quadrature points, the series (three atanh
+// Bound by instruction issue and fixed latencies (62 % of the issue slots at
+// 16 warps per SM).  The quadrature points, the series (three atanh
 // and one atan) and edges 1 and 2 run in pairs through the sm_100 paired FP32
 // instructions; pairing within one (station, facet) needs no more registers
 // than the scalar form, where pairing two stations does.  The vertex sums keep
 // the scalar form's order of additions.  With the adjoints rounded once per
 // station, no range test with library fall-backs and no branch on a
-// lane's adjoints: 264 warp instructions per 32 pairs instead of about 390,
+// lane's adjoints: 250 warp instructions per 32 pairs instead of about 390,
 // both gradient kernels of a 32-body batch (1.29e9 pairs) 18.3 -> 14.6 ms.
 // Four CTAs per SM (128 registers, some spill): three without spill 5 %
 // slower, five 5 %; the facet frame or points in shared memory instead of
